@@ -1767,94 +1767,8 @@ int bfg_particles_info(const bfg_pctx* p, int64_t* n, int* nsteps, int* step_idx
 // library would allocate.  The array exists on every GPU that loads the
 // library, for as long as the library stays loaded.
 
-// per-block partial sums: STATS_BLOCKS blocks x NQ doubles = 370 KiB
+// per-block partial sums: STATS_BLOCKS blocks x NQ doubles = 93 KiB
 static __device__ __align__(256) double g_noalloc_partials[STATS_BLOCKS * NQ];
-
-// same reduction as moments_kernel, over a field stored with a padded row
-// pitch (the reference real layout (nz, ny, nx+2, 3))
-template <typename T>
-__global__ void __launch_bounds__(STATS_THREADS)
-moments_pitched_kernel(const T* __restrict__ r, int nx, int pitch, size_t npts, double me0,
-                       double me1, double me2, double me3, int nbins,
-                       double* __restrict__ partial, unsigned long long* __restrict__ hist) {
-    extern __shared__ unsigned int shist_p[];  // nbins * 4
-    __shared__ double red[STATS_THREADS / 32][NQ];
-    for (int i = threadIdx.x; i < nbins * 4; i += blockDim.x) shist_p[i] = 0;
-    __syncthreads();
-    const double me[4] = {me0, me1, me2, me3};
-    double binsize[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) binsize[i] = 2 * me[i] / nbins;
-    double mn[4] = {0.0, 0.0, 0.0, me3};
-    double mx[4] = {0.0, 0.0, 0.0, 0.0};
-    double sm[8][4];
-#pragma unroll
-    for (int n = 0; n < 8; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) sm[n][i] = 0.0;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < npts;
-         e += (size_t)gridDim.x * blockDim.x) {
-        const size_t x = e % (size_t)nx, rowi = e / (size_t)nx;
-        const T* pt = r + (rowi * (size_t)pitch + x) * 3;
-        double v[4];
-        v[3] = 0.0;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            v[i] = (double)pt[i];
-            v[3] += v[i] * v[i];
-        }
-        v[3] = sqrt(v[3]);
-        {
-            const int b = (int)floor(v[3] * 2 / binsize[3]);
-            if (b >= 0 && b < nbins) atomicAdd(&shist_p[b * 4 + 3], 1u);
-        }
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const int b = (int)floor((v[i] + me[i]) / binsize[i]);
-            if (b >= 0 && b < nbins) atomicAdd(&shist_p[b * 4 + i], 1u);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            mn[i] = fmin(mn[i], v[i]);
-            mx[i] = fmax(mx[i], v[i]);
-            double p = 1.0;
-#pragma unroll
-            for (int n = 0; n < 8; ++n) {
-                p = v[i] * p;
-                sm[n][i] += p;
-            }
-        }
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        double a = warp_min(mn[i]);
-        double b = warp_max(mx[i]);
-        if (lane == 0) {
-            red[wid][0 * 4 + i] = a;
-            red[wid][9 * 4 + i] = b;
-        }
-#pragma unroll
-        for (int n = 0; n < 8; ++n) {
-            double s = warp_sum(sm[n][i]);
-            if (lane == 0) red[wid][(n + 1) * 4 + i] = s;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < NQ) {
-        const int q = threadIdx.x;
-        double acc = red[0][q];
-        for (int w = 1; w < STATS_THREADS / 32; ++w) {
-            const double v = red[w][q];
-            if (q < 4) acc = fmin(acc, v);
-            else if (q >= 36) acc = fmax(acc, v);
-            else acc += v;
-        }
-        partial[(size_t)blockIdx.x * NQ + q] = acc;
-    }
-    for (int i = threadIdx.x; i < nbins * 4; i += blockDim.x)
-        if (shist_p[i]) atomicAdd(&hist[i], (unsigned long long)shist_p[i]);
-}
 
 // Device address of g_noalloc_partials in the current device context.  Host
 // code cannot use the array's name as a device pointer, so the address is
@@ -1938,17 +1852,19 @@ extern "C" int bfg_rspace_stats_noalloc(const void* dev_field, int nx, int ny, i
     }
     const double me3 = max_estimate * std::sqrt(3.0);
     const size_t shmem = (size_t)nbins * 4 * sizeof(unsigned int);
+    const int blocks = stats_blocks(npts);
+    const HistRange range = hist_range(max_estimate, me3, nbins);
     if (real_bytes == 4)
-        moments_pitched_kernel<float><<<STATS_BLOCKS, STATS_THREADS, shmem, s>>>(
-            static_cast<const float*>(dev_field), nx, pitch, npts, max_estimate, max_estimate,
-            max_estimate, me3, nbins, partials, reinterpret_cast<unsigned long long*>(dev_hist));
+        moments_kernel<float><<<blocks, STATS_THREADS, shmem, s>>>(
+            static_cast<const float*>(dev_field), nx, pitch, npts, range, partials,
+            reinterpret_cast<unsigned long long*>(dev_hist));
     else
-        moments_pitched_kernel<double><<<STATS_BLOCKS, STATS_THREADS, shmem, s>>>(
-            static_cast<const double*>(dev_field), nx, pitch, npts, max_estimate, max_estimate,
-            max_estimate, me3, nbins, partials, reinterpret_cast<unsigned long long*>(dev_hist));
+        moments_kernel<double><<<blocks, STATS_THREADS, shmem, s>>>(
+            static_cast<const double*>(dev_field), nx, pitch, npts, range, partials,
+            reinterpret_cast<unsigned long long*>(dev_hist));
     // a failed first launch must not queue the final reduction
     if (cudaGetLastError() != cudaSuccess) return BFG_ECUDA;
-    moments_final<<<1, 64, 0, s>>>(partials, STATS_BLOCKS, 1.0 / (double)npts, dev_moments);
+    moments_final<<<NQ, MOM_FINAL_THREADS, 0, s>>>(partials, blocks, 1.0 / (double)npts, dev_moments);
     if (cudaGetLastError() != cudaSuccess) return BFG_ECUDA;
     return BFG_OK;
 }

@@ -10,7 +10,8 @@ int Engine<T, N>::stats(bfg_ctx* c, int cfield, double max_est, int nbins, doubl
     const size_t spec_n = (size_t)c->nshells * 9;
     // spectrum: SPEC_BLOCKS partials of spec_n doubles, then the result
     int spec_warps = SPEC_WARPS_MAX;
-    while (spec_warps > 1 && (size_t)spec_warps * spec_n * 8 > (size_t)c->smem_optin) --spec_warps;
+    const size_t spec_q = (size_t)c->nshells * SPEC_NQ;  // values per warp
+    while (spec_warps > 1 && (size_t)spec_warps * spec_q * 8 > (size_t)c->smem_optin) --spec_warps;
     if (spec_n * 8 > (size_t)c->smem_optin)
         return fail(c, BFG_EUNSUP, "%d shells do not fit the spectrum kernel's shared memory",
                     c->nshells);
@@ -32,14 +33,14 @@ int Engine<T, N>::stats(bfg_ctx* c, int cfield, double max_est, int nbins, doubl
     const KParams kp = kparams(c, 0.0);
     Prof pr0(c, K_STATS);
     const void* cptr = cfield == B_W0 ? c->w0 : (cfield == B_V1 ? c->v1 : c->wa);
-    const size_t spec_smem = (size_t)spec_warps * spec_n * 8;
+    const size_t spec_smem = (size_t)spec_warps * spec_q * 8;
     CU(ensure_smem(spectrum_kernel<T, N>, spec_smem, c->device));
     spectrum_kernel<T, N><<<SPEC_BLOCKS, spec_warps * 32, spec_smem, c->stream>>>(
         kp, (const C*)cptr, c->nshells, c->dk, d_spart);
     int rc = after_launch(c, "spectrum");
     if (rc) return rc;
-    spectrum_final<<<(unsigned)((spec_n + 255) / 256), 256, 0, c->stream>>>(d_spart, SPEC_BLOCKS,
-                                                                          (int)spec_n, d_spec);
+    spectrum_final<<<(unsigned)((spec_q + 31) / 32), 32 * SPEC_FINAL_GROUPS, 0, c->stream>>>(
+        d_spart, SPEC_BLOCKS, (int)spec_q, d_spec);
     if ((rc = after_launch(c, "spectrum_final"))) return rc;
     // real-space field into v2 (as [z][y][x][3] reals)
     if ((rc = col<CM_IZ_PLAIN>(c, self(c), 1, roles(cfield, B_NONE, B_WB, B_NONE)))) return rc;
@@ -51,10 +52,11 @@ int Engine<T, N>::stats(bfg_ctx* c, int cfield, double max_est, int nbins, doubl
     const size_t npts = (size_t)N * N * N;
     CU(ensure_smem(moments_kernel<T>, (size_t)nbins * 4 * 4, c->device));
     Prof pr1(c, K_STATS);
-    moments_kernel<T><<<STATS_BLOCKS, STATS_THREADS, (size_t)nbins * 4 * 4, c->stream>>>(
-        (const T*)c->v2, npts, max_est, max_est, max_est, me3, nbins, d_part, d_hist);
+    const int mom_blocks = stats_blocks(npts);
+    moments_kernel<T><<<mom_blocks, STATS_THREADS, (size_t)nbins * 4 * 4, c->stream>>>(
+        (const T*)c->v2, N, N, npts, hist_range(max_est, me3, nbins), d_part, d_hist);
     if ((rc = after_launch(c, "moments"))) return rc;
-    moments_final<<<1, 64, 0, c->stream>>>(d_part, STATS_BLOCKS, 1.0 / (double)npts, d_mom);
+    moments_final<<<NQ, MOM_FINAL_THREADS, 0, c->stream>>>(d_part, mom_blocks, 1.0 / (double)npts, d_mom);
     if ((rc = after_launch(c, "moments_final"))) return rc;
     if (spec) CU(cudaMemcpyAsync(spec, d_spec, spec_n * 8, cudaMemcpyDeviceToHost, c->stream));
     if (mom) CU(cudaMemcpyAsync(mom, d_mom, NQ * 8, cudaMemcpyDeviceToHost, c->stream));

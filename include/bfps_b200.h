@@ -320,7 +320,7 @@ int bfg_kernel_launches(const bfg_ctx* ctx, int64_t* count);
  * caller; the work is queued on `stream` (NULL: the default stream) and the
  * call returns without waiting for it.
  *
- * Allocates nothing: the per-block partial sums live in a fixed 370 KiB
+ * Allocates nothing: the per-block partial sums live in a fixed 93 KiB
  * device array inside the library, present on every GPU that loads it until
  * the library is unloaded.  The first call in each device context (and the
  * first after a device reset, which creates a new context) looks up that
