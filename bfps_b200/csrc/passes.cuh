@@ -51,9 +51,11 @@ struct Member {
 };
 enum BufIdx { B_W0 = 0, B_V1 = 1, B_V2 = 2, B_WA = 3, B_WB = 4, B_RU = 5, B_NONE = -1 };
 // which buffers play which part in one launch (B_* indices; rout / rin may
-// also name a complex buffer used as real scratch)
+// also name a complex buffer used as real scratch); user: the caller's array
+// in the reference layout, for the passes that read or write it directly
 struct Roles {
     int in0, in1, out0, out1, v0, vp, fsrc, rout, rin;
+    void* user;
 };
 __host__ __device__ inline Roles roles(int in0, int in1, int out0, int out1, int v0 = B_NONE,
                                        int vp = B_NONE, int fsrc = B_NONE, int rout = B_NONE,
@@ -61,6 +63,7 @@ __host__ __device__ inline Roles roles(int in0, int in1, int out0, int out1, int
     Roles r;
     r.in0 = in0; r.in1 = in1; r.out0 = out0; r.out1 = out1;
     r.v0 = v0; r.vp = vp; r.fsrc = fsrc; r.rout = rout; r.rin = rin;
+    r.user = nullptr;
     return r;
 }
 template <typename T>
@@ -83,6 +86,8 @@ enum ColMode {
     CM_FZ_RK3 = 7,
     CM_FZ_PLAIN = 8,  // W -> S (forward over z)
     CM_IZ_U = 9,      // S -> u^ in W (inverse over kz of compute_velocity)
+    CM_IZ_USER = 10,  // caller's S (rows of N/2 + 1 points) -> W
+    CM_FZ_USER = 11,  // W -> caller's S
 };
 
 __host__ __device__ constexpr int col_nb(int mode) {
@@ -90,7 +95,21 @@ __host__ __device__ constexpr int col_nb(int mode) {
 }
 __host__ __device__ constexpr int col_nbin(int mode) { return mode == CM_Y_INV2 ? 2 : 1; }
 __host__ __device__ constexpr bool col_inverse(int mode) {
-    return mode <= CM_Y_INV1 || mode == CM_IZ_U;
+    return mode <= CM_Y_INV1 || mode == CM_IZ_U || mode == CM_IZ_USER;
+}
+__host__ __device__ constexpr bool col_is_iz(int mode) {
+    return mode == CM_IZ_VEL || mode == CM_IZ_PLAIN || mode == CM_IZ_U || mode == CM_IZ_USER;
+}
+__host__ __device__ constexpr bool col_is_fz(int mode) {
+    return (mode >= CM_FZ_RK1 && mode <= CM_FZ_PLAIN) || mode == CM_FZ_USER;
+}
+// row pitch (complex numbers) of a pass's input and output: the caller's rows
+// hold the N/2 + 1 points of the reference layout, the engine's are padded
+__host__ __device__ constexpr size_t col_pitch_in(int n, int mode) {
+    return (size_t)(mode == CM_IZ_USER ? n / 2 + 1 : n / 2 + 4) * 3;
+}
+__host__ __device__ constexpr size_t col_pitch_out(int n, int mode) {
+    return (size_t)(mode == CM_FZ_USER ? n / 2 + 1 : n / 2 + 4) * 3;
 }
 __host__ __device__ constexpr int pow2floor(int v) {
     return v < 2 ? 1 : 2 * pow2floor(v / 2);
@@ -222,14 +241,14 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
 // global row of tile row l (input side) / lo (output side) for a pass mode
 template <int N, int MODE>
 __device__ __forceinline__ size_t col_in_row(int a, int l) {
-    if (MODE == CM_IZ_VEL || MODE == CM_IZ_PLAIN || MODE == CM_IZ_U) return (size_t)a * N + l;  // S[ky=a][kz=l]
-    if (MODE >= CM_FZ_RK1 && MODE <= CM_FZ_PLAIN) return (size_t)l * N + a;                   // W[z=l][ky=a]
-    return (size_t)a * N + l;                                                                // W[z=a][y=l]
+    if (col_is_iz(MODE)) return (size_t)a * N + l;  // S[ky=a][kz=l]
+    if (col_is_fz(MODE)) return (size_t)l * N + a;  // W[z=l][ky=a]
+    return (size_t)a * N + l;                       // W[z=a][y=l]
 }
 template <int N, int MODE>
 __device__ __forceinline__ size_t col_out_row(int a, int lo) {
-    if (MODE == CM_IZ_VEL || MODE == CM_IZ_PLAIN || MODE == CM_IZ_U) return (size_t)lo * N + a;  // W[z=lo][ky=a]
-    return (size_t)a * N + lo;                                                                 // S or W[z=a]
+    if (col_is_iz(MODE)) return (size_t)lo * N + a;  // W[z=lo][ky=a]
+    return (size_t)a * N + lo;                       // S or W[z=a]
 }
 
 // ---------------------------------------------------------------------------
@@ -401,16 +420,24 @@ __device__ __forceinline__ bool fz_tile_outside(const KParams& kp, int a, int kx
     }
 }
 
+template <typename T, int MODE>
+__device__ __forceinline__ const cpx<T>* col_src(const Member<T>& m, const Roles& rl) {
+    if constexpr (MODE == CM_IZ_USER) return reinterpret_cast<const cpx<T>*>(rl.user);
+    else return mbuf(m, rl.in0);
+}
+
 template <typename T, int N, int MODE, int S>
 __device__ __forceinline__ void col_issue_load(cpx<T>* tile, const cpx<T>* in0,
                                                const cpx<T>* in1, int a, int kx0, int ncol,
-                                               size_t nxp3, int tid) {
+                                               int tid) {
     constexpr int NB = col_nb(MODE);
     constexpr int NBIN = col_nbin(MODE);
     constexpr int TKX = col_tkx<T, N, MODE, S>();
     constexpr int W = 3 * TKX;
     constexpr int PR = col_pitch<T, N, MODE, S>();
-    constexpr int VB = ((W * (int)sizeof(cpx<T>)) % 16 == 0) ? 16 : 8;
+    constexpr size_t PIN = col_pitch_in(N, MODE);
+    // 16-byte copies where every row chunk starts on a 16-byte boundary
+    constexpr int VB = ((W * (int)sizeof(cpx<T>)) % 16 == 0 && PIN * sizeof(cpx<T>) % 16 == 0) ? 16 : 8;
     constexpr int VPE = VB / (int)sizeof(cpx<T>) > 0 ? VB / (int)sizeof(cpx<T>) : 1;  // complex per copy
     constexpr int WV = W / VPE;
     const int nvalid = (3 * ncol + VPE - 1) / VPE;
@@ -420,7 +447,7 @@ __device__ __forceinline__ void col_issue_load(cpx<T>* tile, const cpx<T>* in0,
         const int b = r % NBIN;
         const int l = r / NBIN;
         if (v >= nvalid) continue;
-        const cpx<T>* src = ((b == 0) ? in0 : in1) + col_in_row<N, MODE>(a, l) * nxp3 +
+        const cpx<T>* src = ((b == 0) ? in0 : in1) + col_in_row<N, MODE>(a, l) * PIN +
                             (size_t)kx0 * 3 + v * VPE;
         const int bdst = (MODE == CM_IZ_VEL) ? 1 : b;  // w^ goes to slot 1
         cp_async<VB>(&tile[l * PR + bdst * W + v * VPE], src);
@@ -469,7 +496,7 @@ __device__ __forceinline__ void col_last_store(const cpx<T>* tile, int tid, cons
     constexpr int NST = plan_nstages(N, MR);
     constexpr int R = plan_radix(N, NST - 1, MR);
     constexpr int NW = PP * (N / R);
-    constexpr size_t nxp3 = (size_t)(N / 2 + 4) * 3;
+    constexpr size_t POUT = col_pitch_out(N, MODE);
     const int nval = 3 * ncol;
     for (int w = tid; w < NW; w += NT) {
         const int pn = w % PP;
@@ -481,10 +508,12 @@ __device__ __forceinline__ void col_last_store(const cpx<T>* tile, int tid, cons
         dft<T, INV, R>(v);
         const int bufi = pp / W, q = pp % W;
         if (q >= nval) continue;
-        cpx<T>* dst = mbuf(mb, (bufi == 0) ? rl.out0 : rl.out1) + (size_t)kx0 * 3 + q;
+        cpx<T>* dst = (MODE == CM_FZ_USER ? reinterpret_cast<cpx<T>*>(rl.user)
+                                          : mbuf(mb, (bufi == 0) ? rl.out0 : rl.out1)) +
+                      (size_t)kx0 * 3 + q;
         const int f0 = dif_frequency<N, MR>(bb * R);
 #pragma unroll
-        for (int m = 0; m < R; ++m) dst[col_out_row<N, MODE>(a, f0 + (N / R) * m) * nxp3] = v[m];
+        for (int m = 0; m < R; ++m) dst[col_out_row<N, MODE>(a, f0 + (N / R) * m) * POUT] = v[m];
     }
 }
 
@@ -525,8 +554,8 @@ col_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
         const int m = t / tiles_per, tl = t - m * tiles_per;
         const int kx0 = (tl % ntx) * TKX;
         if (!fz_tile_outside<N, MODE>(mem[m].kp, tl / ntx, kx0))
-            col_issue_load<T, N, MODE, S>(bufs, mbuf(mem[m], rl.in0), mbuf(mem[m], rl.in1), tl / ntx,
-                                          kx0, min(TKX, NXV - kx0), nxp3, tid);
+            col_issue_load<T, N, MODE, S>(bufs, col_src<T, MODE>(mem[m], rl), mbuf(mem[m], rl.in1),
+                                          tl / ntx, kx0, min(TKX, NXV - kx0), tid);
     }
     cp_async_commit();
     __shared__ Member<T> mb;  // this tile's member, read once per tile
@@ -574,9 +603,9 @@ col_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
                 const int mn = tn / tiles_per, tln = tn - mn * tiles_per;
                 const int kx0n = (tln % ntx) * TKX;
                 if (!fz_tile_outside<N, MODE>(mem[mn].kp, tln / ntx, kx0n))
-                    col_issue_load<T, N, MODE, S>(bufs + ((it + 1) & 1) * TILE, mbuf(mem[mn], rl.in0),
+                    col_issue_load<T, N, MODE, S>(bufs + ((it + 1) & 1) * TILE, col_src<T, MODE>(mem[mn], rl),
                                                   mbuf(mem[mn], rl.in1), tln / ntx, kx0n,
-                                                  min(TKX, NXV - kx0n), nxp3, tid);
+                                                  min(TKX, NXV - kx0n), tid);
             }
             cp_async_commit();
         }
@@ -717,8 +746,8 @@ col_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
                 const int mn = tn / tiles_per, tln = tn - mn * tiles_per;
                 const int kx0n = (tln % ntx) * TKX;
                 if (!fz_tile_outside<N, MODE>(mem[mn].kp, tln / ntx, kx0n))
-                    col_issue_load<T, N, MODE, S>(bufs, mbuf(mem[mn], rl.in0), mbuf(mem[mn], rl.in1),
-                                                  tln / ntx, kx0n, min(TKX, NXV - kx0n), nxp3, tid);
+                    col_issue_load<T, N, MODE, S>(bufs, col_src<T, MODE>(mem[mn], rl), mbuf(mem[mn], rl.in1),
+                                                  tln / ntx, kx0n, min(TKX, NXV - kx0n), tid);
             }
             cp_async_commit();
             t = tn;
@@ -848,10 +877,21 @@ __device__ __forceinline__ void r2c_post(const cpx<T>* z, cpx<T>* x, const cpx<T
 // 16-byte vectors.
 template <typename T, int N, int MODE>
 __device__ __forceinline__ void row_issue_load(cpx<T>* stage, const cpx<T>* wu, const cpx<T>* ww,
-                                               const T* rin, size_t row0, int tid) {
+                                               const T* rin, const void* user, size_t row0, int tid) {
     constexpr int ROWS = row_rows<T, N, MODE>();
     constexpr int VPE = 16 / (int)sizeof(cpx<T>);
     if constexpr (MODE == RM_R2C) {
+        if (user) {
+            // the caller's rows of N + 2 points, one pair of values per copy
+            // (8-byte aligned in FP32, 16 in FP64)
+            constexpr int RV = N * 3 / 2, PV = (N + 2) * 3 / 2;
+            const cpx<T>* src = reinterpret_cast<const cpx<T>*>(user) + row0 * PV;
+            for (int e = tid; e < ROWS * RV; e += ROW_THREADS) {
+                const int r = e / RV, v = e - r * RV;
+                cp_async<(int)sizeof(cpx<T>)>(&stage[e], &src[(size_t)r * PV + v]);
+            }
+            return;
+        }
         constexpr int NV = ROWS * N * 3 / 2 / VPE;  // 16-byte vectors of the real rows
         const cpx<T>* src = reinterpret_cast<const cpx<T>*>(rin + row0 * N * 3);
         for (int v = tid; v < NV; v += ROW_THREADS) cp_async16(&stage[v * VPE], &src[v * VPE]);
@@ -902,7 +942,7 @@ row_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
     if (t < ntiles) {
         const int m = t / tiles_per, tl = t - m * tiles_per;
         row_issue_load<T, N, MODE>(stage0, mbuf(mem[m], rl.in0), mbuf(mem[m], rl.in1),
-                                   mreal(mem[m], rl.rin), (size_t)tl * ROWS, tid);
+                                   mreal(mem[m], rl.rin), rl.user, (size_t)tl * ROWS, tid);
     }
     cp_async_commit();
     for (int it = 0; t < ntiles; ++it, t += gridDim.x) {
@@ -912,7 +952,7 @@ row_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
             if (tn < ntiles) {
                 const int mn = tn / tiles_per, tln = tn - mn * tiles_per;
                 row_issue_load<T, N, MODE>(stage0 + ((it + 1) & 1) * STAGE, mbuf(mem[mn], rl.in0),
-                                           mbuf(mem[mn], rl.in1), mreal(mem[mn], rl.rin),
+                                           mbuf(mem[mn], rl.in1), mreal(mem[mn], rl.rin), rl.user,
                                            (size_t)tln * ROWS, tid);
             }
             cp_async_commit();
@@ -921,7 +961,10 @@ row_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
         __syncthreads();
         const int m = t / tiles_per, tl = t - m * tiles_per;
         const size_t row0 = (size_t)tl * ROWS;
-        T* rout = mreal(mem[m], rl.rout);
+        // real rows of N points, or the caller's of N + 2 with the padding zero
+        const bool user_out = MODE == RM_C2R && rl.user;
+        T* rout = user_out ? reinterpret_cast<T*>(rl.user) : mreal(mem[m], rl.rout);
+        const size_t rpitch = user_out ? (size_t)(N + 2) * 3 : (size_t)N * 3;
         cpx<T>* wout = mbuf(mem[m], rl.out0);
 
         if constexpr (MODE == RM_R2C) {
@@ -953,8 +996,11 @@ row_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
                     const int x = r2 % N;
                     const int r = r2 / N;
                     const cpx<T> z = S[(r * 3 + c) * PL + posn[x >> 1]];
-                    rout[(row0 + r) * (N * 3) + x * 3 + c] = (x & 1) ? z.y : z.x;
+                    rout[(row0 + r) * rpitch + x * 3 + c] = (x & 1) ? z.y : z.x;
                 }
+                if (user_out)
+                    for (int e = tid; e < ROWS * 6; e += ROW_THREADS)
+                        rout[(row0 + e / 6) * rpitch + N * 3 + e % 6] = (T)0;
             }
             if constexpr (MODE == RM_C2R) {
                 __syncthreads();

@@ -61,6 +61,5 @@ int Engine<T, N>::stats(bfg_ctx* c, int cfield, double max_est, int nbins, doubl
     if (spec) CU(cudaMemcpyAsync(spec, d_spec, spec_n * 8, cudaMemcpyDeviceToHost, c->stream));
     if (mom) CU(cudaMemcpyAsync(mom, d_mom, NQ * 8, cudaMemcpyDeviceToHost, c->stream));
     if (hist) CU(cudaMemcpyAsync(hist, d_hist, (size_t)nbins * 4 * 8, cudaMemcpyDeviceToHost, c->stream));
-    CU(cudaStreamSynchronize(c->stream));
-    return 0;
+    return finish_call(c);
 }

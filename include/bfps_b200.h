@@ -121,7 +121,10 @@ int bfg_lagrangian_acceleration(bfg_ctx* ctx, void* host);
  * or device memory (unified addressing).  Where either buffer is device
  * memory the call first waits for all work queued on the device (the
  * caller's kernels on any stream), and it returns once the output is
- * complete. */
+ * complete.  Device arrays of the context's GPU that start on 16-byte
+ * boundaries are read and written by the transform itself (the context's
+ * complex velocity is scratch); any other array passes through copies, which
+ * also use the real velocity. */
 int bfg_ift(bfg_ctx* ctx, const void* dev_complex_in, void* dev_real_out);
 int bfg_dft(bfg_ctx* ctx, const void* dev_real_in, void* dev_complex_out);
 

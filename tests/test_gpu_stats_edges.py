@@ -66,8 +66,8 @@ def test_values_on_and_outside_the_bins():
 
 
 def test_nonfinite_values():
-    """Infinities lie outside the histogram and set the extrema; a NaN counts
-    in the first bin and leaves the extrema alone (both as before)."""
+    """Infinities and NaN lie outside the histogram; infinities set the
+    extrema, a NaN leaves them alone."""
     r = np.zeros((1, 1, 4, 3))
     r[0, 0, 1] = [np.inf, -np.inf, np.nan]
     r[0, 0, 2] = [1.0, -2.0, 0.5]
@@ -75,7 +75,7 @@ def test_nonfinite_values():
     assert np.isposinf(mom[9, 0]) and np.isneginf(mom[0, 1])
     assert mom[0, 2] == 0.0 and mom[9, 2] == 0.5
     assert hist[:, 0].sum() == 3 and hist[:, 1].sum() == 3
-    assert hist[0, 2] == 1 and hist[:, 2].sum() == 4
+    assert hist[:, 2].sum() == 3 and hist[:, 3].sum() == 3
 
 
 @pytest.mark.parametrize("n", [16, 64])
