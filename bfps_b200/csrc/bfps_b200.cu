@@ -65,7 +65,13 @@ struct bfg_ctx {
     void* dmember = nullptr;   // this context as a one-element Member<T> array
     std::vector<unsigned char> hmember;  // last uploaded copy
     void* stats_ws = nullptr;  // statistics partial sums
-    int* tctr = nullptr;       // tile counters of the persistent passes (self-resetting)
+    int* tctr = nullptr;       // 16 words: tile counters of the persistent passes (0, 1:
+                               // self-resetting), outside_scan's result (8)
+    // what the passes leave out (passes.cuh, modes outside kM): kx columns and
+    // the bound on |ky| that may hold modes inside; w0_full: the state may hold
+    // modes outside (an upload that did, until it is replaced or low-passed)
+    int pcols = 0, prow = 0;
+    bool w0_full = false;
     unsigned long long* dcount = nullptr;  // bfg_check_finite's counter
     size_t stats_ws_bytes = 0;
     size_t field_bytes = 0;
@@ -220,6 +226,7 @@ static KParams kparams(const bfg_ctx* c, double dt) {
     k.fk1 = c->fk1;
     k.fmode = c->fmode;
     k.dt = dt;
+    k.pcols = c->pcols;
     return k;
 }
 
@@ -364,16 +371,27 @@ struct Engine {
         if (smem > (size_t)c->smem_optin)
             return fail(c, BFG_EUNSUP, "column pass needs %zu bytes of shared memory", smem);
         CU(ensure_smem(kern, smem, c->device));
-        const int ntx = (N / 2 + 1 + TKX - 1) / TKX;
-        const int tiles_per = ntx * N;
+        // the tiles that may hold something: kx columns below pcols, and in the
+        // z passes rows |ky| <= prow
+        const bool part = col_prunes(MODE) && can_prune<T, N>() && (rl.prune & PRUNE_IN);
+        const int ntx = ((part ? c->pcols : N / 2 + 1) + TKX - 1) / TKX;
+        const int kdom = part && (col_is_iz(MODE) || col_fz(MODE)) ? c->prow : -1;
+        const int tiles_per = ntx * (kdom >= 0 ? prune_rows(kdom, N) : N);
         const int ntiles = tiles_per * nmem;
         const int grid = std::min(ntiles, c->nsm * col_ctas<T, N, MODE, S>());
         Prof pr(c, col_kind(MODE));
         // dynamic tile order where a launch has at least 8 tiles per CTA
         int* tctr = ntiles >= 8 * grid ? c->tctr : nullptr;
         kern<<<grid, col_threads<T, N, MODE, S>(), smem, c->stream>>>(mem, rl, (const C*)c->tw, ntx,
-                                                                     tiles_per, ntiles, tctr);
+                                                                     kdom, tiles_per, ntiles, tctr);
         return after_launch(c, "col_pass");
+    }
+
+    // roles of a pass that leaves out what lies outside kM (passes.cuh): `which`
+    // sides of it
+    static Roles pruned(Roles r, int which = PRUNE_IN) {
+        r.prune = which;
+        return r;
     }
 
     // bfg_autotune / bfg_ens_autotune: both schedules of each column pass
@@ -403,9 +421,10 @@ struct Engine {
             *out = f / reps;
             return 0;
         };
-        const Roles r_iz = roles(B_W0, B_NONE, B_WA, B_WB), r_iy = roles(B_WA, B_WB, B_WA, B_WB),
-                    r_fy = roles(B_WA, B_NONE, B_WA, B_NONE),
-                    r_fz = roles(B_WA, B_NONE, B_WB, B_NONE, B_W0, B_V1, B_W0);
+        const Roles r_iz = pruned(roles(B_W0, B_NONE, B_WA, B_WB)),
+                    r_iy = pruned(roles(B_WA, B_WB, B_WA, B_WB)),
+                    r_fy = pruned(roles(B_WA, B_NONE, B_WA, B_NONE)),
+                    r_fz = pruned(roles(B_WA, B_NONE, B_WB, B_NONE, B_W0, B_V1, B_W0));
         int rc;
         if ((rc = time_it([&] { return col_s<CM_IZ_VEL, 0>(c, m, nmem, r_iz); }, &ms[2 * K_IZ]))) return rc;
         if ((rc = time_it([&] { return col_s<CM_IZ_VEL, 1>(c, m, nmem, r_iz); }, &ms[2 * K_IZ + 1]))) return rc;
@@ -520,20 +539,29 @@ struct Engine {
     static int stage(bfg_ctx* c, const Mem* mem, int nmem, int s, bool write_ru) {
         int rc;
         const int src = s == 0 ? B_W0 : (s == 1 ? B_V1 : B_V2);
-        if ((rc = col<CM_IZ_VEL>(c, mem, nmem, roles(src, B_NONE, B_WA, B_WB)))) return rc;
-        if ((rc = col<CM_Y_INV2>(c, mem, nmem, roles(B_WA, B_WB, B_WA, B_WB)))) return rc;
+        // v1 and v2 hold nothing outside kM, the state may (w0_full)
+        const int in = s == 0 && c->w0_full ? 0 : PRUNE_IN;
+        if ((rc = col<CM_IZ_VEL>(c, mem, nmem, pruned(roles(src, B_NONE, B_WA, B_WB), in)))) return rc;
+        if ((rc = col<CM_Y_INV2>(c, mem, nmem, pruned(roles(B_WA, B_WB, B_WA, B_WB), in)))) return rc;
         if (write_ru)
-            rc = row<RM_NONLIN, true>(c, mem, nmem, roles(B_WA, B_WB, B_WA, B_NONE, B_NONE, B_NONE,
-                                                          B_NONE, B_RU));
+            rc = row<RM_NONLIN, true>(c, mem, nmem,
+                                      pruned(roles(B_WA, B_WB, B_WA, B_NONE, B_NONE, B_NONE, B_NONE, B_RU),
+                                             in | PRUNE_OUT));
         else
-            rc = row<RM_NONLIN, false>(c, mem, nmem, roles(B_WA, B_WB, B_WA, B_NONE));
+            rc = row<RM_NONLIN, false>(c, mem, nmem,
+                                       pruned(roles(B_WA, B_WB, B_WA, B_NONE), in | PRUNE_OUT));
         if (rc) return rc;
-        if ((rc = col<CM_Y_FWD1>(c, mem, nmem, roles(B_WA, B_NONE, B_WA, B_NONE)))) return rc;
+        if ((rc = col<CM_Y_FWD1>(c, mem, nmem, pruned(roles(B_WA, B_NONE, B_WA, B_NONE))))) return rc;
         if (s == 0)
-            return col<CM_FZ_RK1>(c, mem, nmem, roles(B_WA, B_NONE, B_V1, B_NONE, B_W0, B_NONE, src));
+            return col<CM_FZ_RK1>(c, mem, nmem,
+                                  pruned(roles(B_WA, B_NONE, B_V1, B_NONE, B_W0, B_NONE, src)));
         if (s == 1)
-            return col<CM_FZ_RK2>(c, mem, nmem, roles(B_WA, B_NONE, B_V2, B_NONE, B_W0, B_V1, src));
-        return col<CM_FZ_RK3>(c, mem, nmem, roles(B_WA, B_NONE, B_W0, B_NONE, B_W0, B_V2, src));
+            return col<CM_FZ_RK2>(c, mem, nmem,
+                                  pruned(roles(B_WA, B_NONE, B_V2, B_NONE, B_W0, B_V1, src)));
+        // a state that is zero outside stays so; one that is not keeps its modes
+        return col<CM_FZ_RK3>(c, mem, nmem,
+                              pruned(roles(B_WA, B_NONE, B_W0, B_NONE, B_W0, B_V2, src),
+                                     c->w0_full ? 0 : PRUNE_IN));
     }
 
     static int finish_step(bfg_ctx* c, const Mem* mem, int nmem) {
@@ -555,10 +583,17 @@ struct Engine {
 
     static int velocity_rspace(bfg_ctx* c) {
         int rc;
-        if ((rc = col<CM_IZ_U>(c, self(c), 1, roles(B_W0, B_NONE, B_WB, B_NONE)))) return rc;
-        if ((rc = col<CM_Y_INV1>(c, self(c), 1, roles(B_WB, B_NONE, B_WB, B_NONE)))) return rc;
-        return row<RM_C2R, false>(c, self(c), 1, roles(B_WB, B_NONE, B_NONE, B_NONE, B_NONE, B_NONE,
-                                                       B_NONE, B_RU));
+        // u^ is zero outside kM whatever the state holds
+        if ((rc = col<CM_IZ_U>(c, self(c), 1, pruned(roles(B_W0, B_NONE, B_WB, B_NONE))))) return rc;
+        return rspace(c, B_WB, B_RU, PRUNE_IN);
+    }
+    // the y and x passes to real space of a complex work buffer: reals to `to`
+    static int rspace(bfg_ctx* c, int buf, int to, int prune) {
+        int rc = col<CM_Y_INV1>(c, self(c), 1, pruned(roles(buf, B_NONE, buf, B_NONE), prune));
+        if (rc) return rc;
+        return row<RM_C2R, false>(
+            c, self(c), 1,
+            pruned(roles(buf, B_NONE, B_NONE, B_NONE, B_NONE, B_NONE, B_NONE, to), prune));
     }
 
     static int fixup(bfg_ctx* c) {
@@ -671,10 +706,9 @@ struct Engine {
     static int acceleration_rspace(bfg_ctx* c) {
         int rc;
         if ((rc = acceleration(c))) return rc;
-        if ((rc = col<CM_IZ_PLAIN>(c, self(c), 1, roles(B_WB, B_NONE, B_WA, B_NONE)))) return rc;
-        if ((rc = col<CM_Y_INV1>(c, self(c), 1, roles(B_WA, B_NONE, B_WA, B_NONE)))) return rc;
-        return row<RM_C2R, false>(c, self(c), 1, roles(B_WA, B_NONE, B_NONE, B_NONE, B_NONE, B_NONE,
-                                                       B_NONE, B_V2));
+        // zero outside kM
+        if ((rc = col<CM_IZ_PLAIN>(c, self(c), 1, pruned(roles(B_WB, B_NONE, B_WA, B_NONE))))) return rc;
+        return rspace(c, B_WA, B_V2, PRUNE_IN);
     }
 
     static int stats(bfg_ctx* c, int cfield, double max_est, int nbins, double* spec, double* mom,
@@ -713,6 +747,15 @@ static int dispatch(bfg_ctx* c, Args... args) {
 template <typename T, int N>
 struct OpStep {
     static int run(bfg_ctx* c, double dt, bfg_pctx* p);
+};
+// set_prune: what the passes of this grid leave out
+template <typename T, int N>
+struct OpPrune {
+    static int run(bfg_ctx* c) {
+        c->pcols = can_prune<T, N>() ? prune_cols(c->kM2, c->dkx, N, col_pblk<T, N>()) : N / 2 + 1;
+        c->prow = std::max(prune_k(c->kM2, c->kM2, c->dky, N), 0);
+        return 0;
+    }
 };
 template <typename T, int N>
 struct OpVelocity {
@@ -1043,6 +1086,29 @@ int OpStep<T, N>::run(bfg_ctx* c, double dt, bfg_pctx* p) {
     return E::finish_step(c, E::self(c), 1);
 }
 
+// sets *found where a state-layout field holds a value other than zero at a mode
+// outside kM (one warp per row; the modes inside are not read)
+template <typename T>
+__global__ void outside_scan(const KParams kp, const cpx<T>* __restrict__ w, int N,
+                             int* __restrict__ found) {
+    const int lane = threadIdx.x & 31;
+    const int nw = gridDim.x * (blockDim.x >> 5);
+    bool any = false;
+    for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < N * N; r += nw) {
+        const int iy = r / N, iz = r - iy * N;
+        const double ky = kp.dky * (double)(iy <= N / 2 ? iy : iy - N);
+        const double kz = kp.dkz * (double)(iz <= N / 2 ? iz : iz - N);
+        for (int ix = lane; ix < kp.nxv; ix += 32) {
+            const double kx = ix * kp.dkx;
+            if ((kx * kx + ky * ky) + kz * kz <= kp.kM2) continue;
+            const cpx<T>* a = w + ((size_t)r * kp.nxp + ix) * 3;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) any = any || a[c].x != (T)0 || a[c].y != (T)0;
+        }
+    }
+    if (any) *found = 1;
+}
+
 // ================================================================ ABI ==
 extern "C" {
 
@@ -1144,6 +1210,7 @@ int bfg_ctx_create(bfg_ctx** out, int nx, int ny, int nz, double dkx, double dky
     if (cudaMalloc(&c->fac, 3 * (size_t)(c->nxv + 2 * nx) * real_bytes) != cudaSuccess)
         return bail(BFG_ENOMEM);
     if ((rc = upload_tables(c))) return bail(rc);
+    if ((rc = dispatch<OpPrune>(c))) return bail(rc);
     *out = c;
     return BFG_OK;
 }
@@ -1220,6 +1287,22 @@ static int field_copy(bfg_ctx* c, int field_id, void* host, bool upload) {
         pitch_copy8<<<grid, 256, 0, c->stream>>>((const uint2*)c->wb, hpitch / 8, (uint2*)dev,
                                                  dpitch / 8, wq, 0, rows);
         CU(cudaGetLastError());
+        if (field_id == BFG_FIELD_VORTICITY) {
+            int* found = c->tctr + 8;
+            int h = 1;
+            c->w0_full = true;
+            CU(cudaMemsetAsync(found, 0, sizeof(int), c->stream));
+            if (c->real_bytes == 4)
+                outside_scan<float><<<grid, 256, 0, c->stream>>>(kparams(c, 0.0), (const cpx<float>*)dev,
+                                                                 c->n, found);
+            else
+                outside_scan<double><<<grid, 256, 0, c->stream>>>(kparams(c, 0.0),
+                                                                  (const cpx<double>*)dev, c->n, found);
+            CU(cudaGetLastError());
+            CU(cudaMemcpyAsync(&h, found, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+            CU(cudaStreamSynchronize(c->stream));
+            c->w0_full = h != 0;
+        }
     } else {
         pitch_copy8<<<grid, 256, 0, c->stream>>>((const uint2*)dev, dpitch / 8, (uint2*)c->wb,
                                                  hpitch / 8, wq, (int)((hpitch - width) / 8), rows);
@@ -1245,6 +1328,7 @@ int bfg_read_checkpoint_fixup(bfg_ctx* c) {
     rc = dispatch<OpFixup>(c);
     if (rc) return rc;
     CU(cudaStreamSynchronize(c->stream));
+    c->w0_full = false;  // low-passed
     return 0;
 }
 
@@ -1480,6 +1564,7 @@ int bfg_ctx_reset(bfg_ctx* c) {
         CU(cudaMemsetAsync(b, 0, c->field_bytes, c->stream));
     c->iteration = 0;
     CU(cudaStreamSynchronize(c->stream));
+    c->w0_full = false;
     return 0;
 }
 
@@ -2171,6 +2256,13 @@ static int ens_prepare(bfg_ens* e) {
         g->launcher.real_bytes = c0->real_bytes;
         g->launcher.device = c0->device;
         g->launcher.tw = c0->tw;
+        // the launches cover what any member holds
+        for (int i : g->members) {
+            const bfg_ctx* ci = e->entries[i].ctx;
+            g->launcher.pcols = std::max(g->launcher.pcols, ci->pcols);
+            g->launcher.prow = std::max(g->launcher.prow, ci->prow);
+            g->launcher.w0_full = g->launcher.w0_full || ci->w0_full;
+        }
         e->groups.push_back(g);
         if (cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&g->ev_s1, cudaEventDisableTiming) != cudaSuccess ||
@@ -2346,6 +2438,14 @@ int bfg_ens_step(bfg_ens* e, int nsteps) {
     if (!e || nsteps < 0) return BFG_EINVAL;
     if (e->entries.empty()) return 0;
     cudaSetDevice(e->device);
+    // a member's state was replaced since the graphs were captured by one that
+    // holds modes outside kM (or no longer does)
+    for (EnsGroup* g : e->groups) {
+        bool full = false;
+        for (size_t k = 0; !e->dirty && k < g->members.size(); ++k)
+            full = full || e->entries[g->members[k]].ctx->w0_full;
+        if (full != g->launcher.w0_full) e->dirty = true;
+    }
     int rc = ens_prepare(e);
     if (rc) return rc;
     // e->stream carries the tracers and orders the call: it starts the

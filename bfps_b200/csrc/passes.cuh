@@ -36,6 +36,7 @@ struct KParams {
     double famp, fk0, fk1;
     int fmode;
     double dt;
+    int pcols;         // kx columns that may hold modes inside kM (prune_cols)
 };
 
 // One DNS instance as the kernels see it: parameters, its five complex
@@ -56,6 +57,7 @@ enum BufIdx { B_W0 = 0, B_V1 = 1, B_V2 = 2, B_WA = 3, B_WB = 4, B_RU = 5, B_NONE
 struct Roles {
     int in0, in1, out0, out1, v0, vp, fsrc, rout, rin;
     void* user;
+    int prune;  // PRUNE_IN / PRUNE_OUT (see "modes outside kM" below)
 };
 __host__ __device__ inline Roles roles(int in0, int in1, int out0, int out1, int v0 = B_NONE,
                                        int vp = B_NONE, int fsrc = B_NONE, int rout = B_NONE,
@@ -64,6 +66,7 @@ __host__ __device__ inline Roles roles(int in0, int in1, int out0, int out1, int
     r.in0 = in0; r.in1 = in1; r.out0 = out0; r.out1 = out1;
     r.v0 = v0; r.vp = vp; r.fsrc = fsrc; r.rout = rout; r.rin = rin;
     r.user = nullptr;
+    r.prune = 0;
     return r;
 }
 template <typename T>
@@ -197,6 +200,95 @@ __host__ __device__ constexpr int col_pitch() {
 template <typename T, int N, int MODE, int S>
 __host__ __device__ constexpr size_t col_smem_bytes() {
     return col_bytes_nb<T, N, MODE>(col_tkx<T, N, MODE, S>(), col_nbuf<T, N, MODE, S>());
+}
+
+// ---- modes outside kM -------------------------------------------------------
+// u^ is zero outside the sphere |k| <= kM, and so are the RK stage states v1,
+// v2 and (unless the caller uploaded something else: bfg_ctx::w0_full) the
+// state.  So the passes of a step neither store nor read what lies outside:
+//   state layout (v1, v2; w0 where it is known to be zero outside): kz rows of
+//     a (ky, kx block) beyond prune_k(kM^2 - kx^2 - ky^2, dkz);
+//   work layout between the z and y passes: ky rows of a kx block beyond
+//     prune_k(kM^2 - kx^2, dky);
+//   work layout around the x pass: kx columns from prune_cols on.
+// kx is the first column of its block of col_pblk columns, a multiple of every
+// tile width of the grid, so all passes and both schedules agree on what
+// exists; a column (row) that exists has at least the row 0, whatever the
+// rounding; prune_k errs on the large side, so nothing inside the sphere is
+// lost.  Grids whose tiles span whole rows (N <= 64) are not pruned: they fit
+// in L2 and are bound by latency.  With the smooth filter (kM = N/2 - 1) a
+// column pass keeps 79 % of its (kx, ky) columns, with the two-thirds rule
+// (kM = N/3 - 1) 35 %.  Per launch, 512^3 FP32, smooth: IZ 1319 -> 1095, IY 1424
+// -> 1324, FZ 1568 -> 1162 us; 256^3 FP64, two thirds: IZ 317 -> 124, IY 334 ->
+// 217, FY 169 -> 119, FZ 218 -> 112 us.
+enum { PRUNE_IN = 1, PRUNE_OUT = 2 };
+template <typename T, int N, int MODE>
+__host__ __device__ constexpr int col_tkx_max() {
+    return col_tkx<T, N, MODE, 0>() > col_tkx<T, N, MODE, 1>() ? col_tkx<T, N, MODE, 0>()
+                                                              : col_tkx<T, N, MODE, 1>();
+}
+__host__ __device__ constexpr int max4(int a, int b, int c, int d) {
+    return (a > b ? a : b) > (c > d ? c : d) ? (a > b ? a : b) : (c > d ? c : d);
+}
+template <typename T, int N>
+__host__ __device__ constexpr int col_pblk() {
+    return max4(max4(col_tkx_max<T, N, CM_IZ_VEL>(), col_tkx_max<T, N, CM_IZ_U>(),
+                     col_tkx_max<T, N, CM_Y_INV1>(), col_tkx_max<T, N, CM_Y_INV2>()),
+                max4(col_tkx_max<T, N, CM_IZ_PLAIN>(), col_tkx_max<T, N, CM_Y_FWD1>(), 0, 0),
+                col_tkx_max<T, N, CM_FZ_RK1>(),
+                max4(col_tkx_max<T, N, CM_FZ_RK2>(), col_tkx_max<T, N, CM_FZ_RK3>(), 0, 0));
+}
+template <typename T, int N>
+__host__ __device__ constexpr bool can_prune() { return col_pblk<T, N>() < N / 2 + 1; }
+__host__ __device__ constexpr bool col_prunes(int mode) {
+    return mode == CM_IZ_VEL || mode == CM_IZ_U || mode == CM_IZ_PLAIN || mode == CM_Y_INV1 ||
+           mode == CM_Y_INV2 || mode == CM_Y_FWD1 || col_fz(mode);
+}
+// largest index k >= 0 that may satisfy (k dk)^2 <= room, at most n / 2; -1 if
+// none does
+__host__ __device__ inline int prune_k(double room, double scale, double dk, int n) {
+    if (room < -1e-9 * scale) return -1;
+    const double k = sqrt(room > 0.0 ? room : 0.0) / dk * (1.0 + 1e-9) + 1e-4;
+    return k < n / 2 ? (int)k : n / 2;
+}
+// rows with |index| <= k of n in wrapped order, and row r of them
+__host__ __device__ inline int prune_rows(int k, int n) { return 2 * k + 1 < n ? 2 * k + 1 : n; }
+__host__ __device__ inline int prune_row(int r, int k, int n) {
+    return r <= k ? r : r + n - prune_rows(k, n);
+}
+// kx columns that may hold something
+__host__ __device__ inline int prune_cols(double kM2, double dkx, int n, int blk) {
+    const int c = (prune_k(kM2, kM2, dkx, n) / blk + 1) * blk;
+    return c < n / 2 + 1 ? c : n / 2 + 1;
+}
+// ky bound of the block of column kx0 (-1: the block does not exist)
+template <typename T, int N>
+__device__ __forceinline__ int prune_ky(const KParams& kp, int kx0) {
+    constexpr int B = col_pblk<T, N>();
+    if (kx0 >= kp.pcols) return -1;
+    const double kx = (double)(kx0 / B * B) * kp.dkx;
+    return max(prune_k(kp.kM2 - kx * kx, kp.kM2, kp.dky, N), 0);
+}
+// kz bound of the block of column kx0 and row ky = a (-1: they do not exist)
+template <typename T, int N>
+__device__ __forceinline__ int prune_kz(const KParams& kp, int kx0, int a) {
+    constexpr int B = col_pblk<T, N>();
+    const int ia = a <= N / 2 ? a : N - a;
+    if (ia > prune_ky<T, N>(kp, kx0)) return -1;
+    const double kx = (double)(kx0 / B * B) * kp.dkx, ky = kp.dky * (double)ia;
+    return max(prune_k(kp.kM2 - kx * kx - ky * ky, kp.kM2, kp.dkz, N), 0);
+}
+// rows along l that the tile (a, kx0) of a pass holds (bound on |l|; N / 2:
+// all of them, -1: the tile is empty)
+template <typename T, int N, int MODE>
+__device__ __forceinline__ int tile_bound(const KParams& kp, const Roles& rl, int a, int kx0) {
+    if constexpr (col_prunes(MODE) && can_prune<T, N>()) {
+        if (!(rl.prune & PRUNE_IN)) return N / 2;
+        if constexpr (col_is_iz(MODE) || col_fz(MODE)) return prune_kz<T, N>(kp, kx0, a);
+        else return prune_ky<T, N>(kp, kx0);
+    } else {
+        return N / 2;
+    }
 }
 
 template <int N>
@@ -429,7 +521,7 @@ __device__ __forceinline__ const cpx<T>* col_src(const Member<T>& m, const Roles
 template <typename T, int N, int MODE, int S>
 __device__ __forceinline__ void col_issue_load(cpx<T>* tile, const cpx<T>* in0,
                                                const cpx<T>* in1, int a, int kx0, int ncol,
-                                               int tid) {
+                                               int kb, int tid) {
     constexpr int NB = col_nb(MODE);
     constexpr int NBIN = col_nbin(MODE);
     constexpr int TKX = col_tkx<T, N, MODE, S>();
@@ -441,16 +533,29 @@ __device__ __forceinline__ void col_issue_load(cpx<T>* tile, const cpx<T>* in0,
     constexpr int VPE = VB / (int)sizeof(cpx<T>) > 0 ? VB / (int)sizeof(cpx<T>) : 1;  // complex per copy
     constexpr int WV = W / VPE;
     const int nvalid = (3 * ncol + VPE - 1) / VPE;
-    for (int e = tid; e < N * NBIN * WV; e += col_threads<T, N, MODE, S>()) {
+    // rows |l| <= kb hold the input of an inverse pass, the others are zero
+    // (the input of a forward pass lies in real space along l: all rows)
+    constexpr bool PR_IN = col_prunes(MODE) && can_prune<T, N>() && col_inverse(MODE);
+    const int nl = PR_IN ? prune_rows(kb, N) : N;
+    for (int e = tid; e < nl * NBIN * WV; e += col_threads<T, N, MODE, S>()) {
         const int v = e % WV;
         const int r = e / WV;
         const int b = r % NBIN;
-        const int l = r / NBIN;
+        const int l = PR_IN ? prune_row(r / NBIN, kb, N) : r / NBIN;
         if (v >= nvalid) continue;
         const cpx<T>* src = ((b == 0) ? in0 : in1) + col_in_row<N, MODE>(a, l) * PIN +
                             (size_t)kx0 * 3 + v * VPE;
         const int bdst = (MODE == CM_IZ_VEL) ? 1 : b;  // w^ goes to slot 1
         cp_async<VB>(&tile[l * PR + bdst * W + v * VPE], src);
+    }
+    if constexpr (PR_IN) {
+        // whole rows of both buffers (u^ beside w^ included)
+        constexpr int WZ = NB * W;
+        const int nz = N - nl;
+        for (int e = tid; e < nz * WZ; e += col_threads<T, N, MODE, S>()) {
+            const int r = e / WZ;
+            tile[(kb + 1 + r) * PR + e - r * WZ] = zero_c<T>();
+        }
     }
 }
 
@@ -486,7 +591,7 @@ __device__ __forceinline__ void tile_tickets_done(int* tctr, int tid) {
 // holds the Nyquist column only and PP counts its pencils (3 per buffer).
 template <typename T, int N, int MODE, int S, int PP, bool NYQ>
 __device__ __forceinline__ void col_last_store(const cpx<T>* tile, int tid, const Member<T>& mb,
-                                               const Roles& rl, int a, int kx0, int ncol) {
+                                               const Roles& rl, int a, int kx0, int ncol, int kb) {
     constexpr int NT = col_threads<T, N, MODE, S>();
     constexpr int TKX = col_tkx<T, N, MODE, S>();
     constexpr int W = 3 * TKX;
@@ -513,14 +618,19 @@ __device__ __forceinline__ void col_last_store(const cpx<T>* tile, int tid, cons
                       (size_t)kx0 * 3 + q;
         const int f0 = dif_frequency<N, MR>(bb * R);
 #pragma unroll
-        for (int m = 0; m < R; ++m) dst[col_out_row<N, MODE>(a, f0 + (N / R) * m) * POUT] = v[m];
+        for (int m = 0; m < R; ++m) {
+            const int f = f0 + (N / R) * m;
+            // a forward y pass keeps the ky rows that the z pass reads
+            if (MODE == CM_Y_FWD1 && can_prune<T, N>() && (f <= N / 2 ? f : N - f) > kb) continue;
+            dst[col_out_row<N, MODE>(a, f) * POUT] = v[m];
+        }
     }
 }
 
 template <typename T, int N, int MODE, int S>
 __global__ void __launch_bounds__(col_threads<T, N, MODE, S>(), col_ctas<T, N, MODE, S>())
 col_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __restrict__ tw_g,
-         int ntx, int tiles_per, int ntiles, int* __restrict__ tctr) {
+         int ntx, int kdom, int tiles_per, int ntiles, int* __restrict__ tctr) {
     constexpr int NT = col_threads<T, N, MODE, S>();
     constexpr int NBUF = col_nbuf<T, N, MODE, S>();
     constexpr int NB = col_nb(MODE);
@@ -540,28 +650,45 @@ col_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
     for (int i = tid; i < N; i += NT) tw[i] = tw_g[i];
 
     // tile t: member t / tiles_per, then (a, kx-tile) with the kx-tile fastest
-    // tiles: this one (t) and, with two buffers, the next one (tnext)
-    __shared__ int s_tk[2];
+    // (ntx kx-tiles; rows a with |a| <= kdom where kdom >= 0, else all).
+    // Tiles: this one (t) and, with two buffers, the next one (tnext), each with
+    // its bound on |l| (kb, kbnext); thread 0 draws them, works out the bound
+    // once for the block and passes over the empty ones.
+    __shared__ int2 s_tk[2];
     int nk = 0;  // tickets drawn (thread 0)
+    auto row_of = [&](int r) { return kdom >= 0 ? prune_row(r, kdom, N) : r; };
+    auto draw = [&]() {
+        for (;;) {
+            const int tt = tile_ticket(tctr, nk++);
+            if (tt >= ntiles) return make_int2(tt, -1);
+            const int m = tt / tiles_per, tl = tt - m * tiles_per;
+            const int b = tile_bound<T, N, MODE>(mem[m].kp, rl, row_of(tl / ntx), (tl % ntx) * TKX);
+            if (b >= 0) return make_int2(tt, b);
+        }
+    };
+    auto load = [&](int tt, int b, cpx<T>* dst) {
+        const int m = tt / tiles_per, tl = tt - m * tiles_per;
+        const int a = row_of(tl / ntx), kx0 = (tl % ntx) * TKX;
+        if (!fz_tile_outside<N, MODE>(mem[m].kp, a, kx0))
+            col_issue_load<T, N, MODE, S>(dst, col_src<T, MODE>(mem[m], rl), mbuf(mem[m], rl.in1), a,
+                                          kx0, min(TKX, NXV - kx0), b, tid);
+    };
     if (tid == 0) {
-        s_tk[0] = tile_ticket(tctr, nk++);
-        s_tk[1] = NBUF == 2 ? tile_ticket(tctr, nk++) : 0;
+        s_tk[0] = draw();
+        s_tk[1] = NBUF == 2 ? draw() : make_int2(0, 0);
     }
     __syncthreads();
-    int t = s_tk[0];
-    int tnext = s_tk[1];
-    if (t < ntiles) {
-        const int m = t / tiles_per, tl = t - m * tiles_per;
-        const int kx0 = (tl % ntx) * TKX;
-        if (!fz_tile_outside<N, MODE>(mem[m].kp, tl / ntx, kx0))
-            col_issue_load<T, N, MODE, S>(bufs, col_src<T, MODE>(mem[m], rl), mbuf(mem[m], rl.in1),
-                                          tl / ntx, kx0, min(TKX, NXV - kx0), tid);
-    }
+    int t = s_tk[0].x, kb = s_tk[0].y;
+    int tnext = s_tk[1].x, kbnext = s_tk[1].y;
+    if (t < ntiles) load(t, kb, bufs);
     cp_async_commit();
     __shared__ Member<T> mb;  // this tile's member, read once per tile
     for (int it = 0; t < ntiles; ++it) {
         cpx<T>* tile = bufs + (NBUF == 2 ? (it & 1) * TILE : 0);
         const int m = t / tiles_per, tl = t - m * tiles_per;
+        const int a = row_of(tl / ntx);
+        const int kx0 = (tl % ntx) * TKX;
+        const int nl = prune_rows(kb, N);  // rows along l that exist in k space
         {
             // the previous tile ended with a barrier: nobody reads mb now
             constexpr int NWORDS = (int)(sizeof(Member<T>) / sizeof(int));
@@ -572,10 +699,8 @@ col_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
         if constexpr (NRK > 0) {
             // RK operands of this tile, rows S[ky=a][kz=l][kx0..kx0+TKX): into
             // L2 while the tile is transformed, read by the epilogue; only
-            // rows with a mode inside kM2, except v0 in stage 3, which the
-            // epilogue also reads outside
-            const int a = tl / ntx;
-            const int kx0 = (tl % ntx) * TKX;
+            // rows with a mode inside kM2, except v0 in stage 3 on a state
+            // that is not zero outside, which the epilogue also reads there
             const cpx<T>* rk_v0 = mbuf(mem[m], rl.v0);  // mb is not yet visible to all
             const cpx<T>* rk_vp = NRK > 1 ? mbuf(mem[m], rl.vp) : rk_v0;
             const KParams& gkp = mem[m].kp;
@@ -583,11 +708,11 @@ col_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
             const double room = gkp.kM2 - (kxv * kxv + kyv * kyv);  // kz^2 left inside
             constexpr int LINES = (3 * TKX * (int)sizeof(cpx<T>) + 127) / 128 + 1;
             const int nbytes = 3 * min(TKX, NXV - kx0) * (int)sizeof(cpx<T>);
-            for (int e = tid; e < N * NRK * LINES; e += NT) {
+            for (int e = tid; e < nl * NRK * LINES; e += NT) {
                 const int q = e % LINES;
                 const int r = e / LINES;
                 const int arr = r % NRK;
-                const int l = r / NRK;
+                const int l = prune_row(r / NRK, kb, N);
                 const double kz = kwrap<N>(l, gkp.dkz);
                 const bool used = (MODE == CM_FZ_RK3 && arr == 0) || kz * kz <= room;
                 if (!used) continue;
@@ -598,15 +723,7 @@ col_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
         }
         if constexpr (NBUF == 2) {
             // the next tile streams into the other buffer while this one is transformed
-            const int tn = tnext;
-            if (tn < ntiles) {
-                const int mn = tn / tiles_per, tln = tn - mn * tiles_per;
-                const int kx0n = (tln % ntx) * TKX;
-                if (!fz_tile_outside<N, MODE>(mem[mn].kp, tln / ntx, kx0n))
-                    col_issue_load<T, N, MODE, S>(bufs + ((it + 1) & 1) * TILE, col_src<T, MODE>(mem[mn], rl),
-                                                  mbuf(mem[mn], rl.in1), tln / ntx, kx0n,
-                                                  min(TKX, NXV - kx0n), tid);
-            }
+            if (tnext < ntiles) load(tnext, kbnext, bufs + ((it + 1) & 1) * TILE);
             cp_async_commit();
         }
         if constexpr (NBUF == 2) cp_async_wait<1>();
@@ -614,9 +731,7 @@ col_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
         __syncthreads();
         // ticket for the tile after the prefetched one (two buffers) or for
         // the next one (one buffer); read after the barrier ending this tile
-        if (tid == 0) s_tk[0] = tile_ticket(tctr, nk++);
-        const int a = tl / ntx;
-        const int kx0 = (tl % ntx) * TKX;
+        if (tid == 0) s_tk[0] = draw();
         const int ncol = min(TKX, NXV - kx0);
         const KParams& kp = mb.kp;
 
@@ -676,12 +791,13 @@ col_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
                 if (col < ncol) {
                     const double kx = (double)(kx0 + col) * kp.dkx;
                     const double kxy2 = kx * kx + ky * ky;
-                    for (int l = l0; l < N; l += NT / TKX) point(col, l, kxy2, (T)kx, (T)ky);
+                    for (int r = l0; r < nl; r += NT / TKX)
+                        point(col, prune_row(r, kb, N), kxy2, (T)kx, (T)ky);
                 }
             } else {
-                for (int e = tid; e < N * TKX; e += NT) {
+                for (int e = tid; e < nl * TKX; e += NT) {
                     const int col = e % TKX;
-                    const int l = e / TKX;
+                    const int l = prune_row(e / TKX, kb, N);
                     if (col >= ncol) continue;
                     const double kx = (double)(kx0 + col) * kp.dkx;
                     point(col, l, kx * kx + ky * ky, (T)kx, (T)ky);
@@ -720,12 +836,12 @@ col_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
                 const int col = tid % TKX;
                 if (col < ncol) {
                     const FzCol<T> fc = fz_col<T, N, MODE>(kp, mb.fac, a, kx0 + col, ky);
-                    for (int l = tid / TKX; l < N; l += NT / TKX) mode(col, l, fc);
+                    for (int r = tid / TKX; r < nl; r += NT / TKX) mode(col, prune_row(r, kb, N), fc);
                 }
             } else {
-                for (int e = tid; e < N * TKX; e += NT) {
+                for (int e = tid; e < nl * TKX; e += NT) {
                     const int col = e % TKX;
-                    const int l = e / TKX;
+                    const int l = prune_row(e / TKX, kb, N);
                     if (col >= ncol) continue;
                     mode(col, l, fz_col<T, N, MODE>(kp, mb.fac, a, kx0 + col, ky));
                 }
@@ -733,28 +849,24 @@ col_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
         } else {
             if (ncol == TKX) {
                 dif_range<T, N, 0, NST - 1, INV, P, LY, 1, N, MR>(tile, tw, tid, NT);
-                col_last_store<T, N, MODE, S, P, false>(tile, tid, mb, rl, a, kx0, ncol);
+                col_last_store<T, N, MODE, S, P, false>(tile, tid, mb, rl, a, kx0, ncol, kb);
             } else {
                 dif_range<T, N, 0, NST - 1, INV, PN, LYN, 1, N, MR>(tile, tw, tid, NT);
-                col_last_store<T, N, MODE, S, PN, true>(tile, tid, mb, rl, a, kx0, ncol);
+                col_last_store<T, N, MODE, S, PN, true>(tile, tid, mb, rl, a, kx0, ncol, kb);
             }
         }
         __syncthreads();  // this buffer is refilled by the next load
         if constexpr (NBUF == 1) {
-            const int tn = s_tk[0];
-            if (tn < ntiles) {
-                const int mn = tn / tiles_per, tln = tn - mn * tiles_per;
-                const int kx0n = (tln % ntx) * TKX;
-                if (!fz_tile_outside<N, MODE>(mem[mn].kp, tln / ntx, kx0n))
-                    col_issue_load<T, N, MODE, S>(bufs, col_src<T, MODE>(mem[mn], rl), mbuf(mem[mn], rl.in1),
-                                                  tln / ntx, kx0n, min(TKX, NXV - kx0n), tid);
-            }
+            t = s_tk[0].x;
+            kb = s_tk[0].y;
+            if (t < ntiles) load(t, kb, bufs);
             cp_async_commit();
-            t = tn;
         } else {
-            const int t2 = s_tk[0];
+            const int2 t2 = s_tk[0];
             t = tnext;
-            tnext = t2;
+            kb = kbnext;
+            tnext = t2.x;
+            kbnext = t2.y;
         }
     }
     cp_async_wait<0>();
@@ -813,16 +925,18 @@ __host__ __device__ constexpr size_t row_smem_bytes() {
 
 // C2R pre-processing (pairs k, M-k; X[0] and X[M] enter with their real
 // parts only), reading X from an interleaved row (stride 3) and writing Z to
-// a contiguous pencil.
+// a contiguous pencil; columns from kin on are zero and not read.
 template <typename T, int N>
-__device__ __forceinline__ void c2r_pre(const cpx<T>* x, cpx<T>* z, const cpx<T>* tw, int k) {
+__device__ __forceinline__ void c2r_pre(const cpx<T>* x, cpx<T>* z, const cpx<T>* tw, int k,
+                                        int kin) {
     constexpr int M = N / 2;
     if (k == 0) {
-        const T x0 = x[0].x, xm = x[3 * M].x;
+        const T x0 = x[0].x, xm = M < kin ? x[3 * M].x : (T)0;
         z[0] = mk<T>(x0 + xm, x0 - xm);
         return;
     }
-    const cpx<T> a = x[3 * k], b = x[3 * (M - k)];
+    const cpx<T> a = k < kin ? x[3 * k] : zero_c<T>();
+    const cpx<T> b = M - k < kin ? x[3 * (M - k)] : zero_c<T>();
     const cpx<T> w = tw[k];  // exp(-2 pi i k / N)
     // Z[k] = (a + conj b) + i conj(w) (a - conj b)
     {
@@ -980,10 +1094,11 @@ row_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
             __syncthreads();
         } else {
             // C2R pre-processing, interleaved rows -> pencils
+            const int kin = can_prune<T, N>() && (rl.prune & PRUNE_IN) ? mem[m].kp.pcols : M + 1;
             for (int e = tid; e < NP * (M / 2 + 1); e += ROW_THREADS) {
                 const int k = e % (M / 2 + 1);
                 const int p = e / (M / 2 + 1);  // = (b*ROWS + r)*3 + c
-                c2r_pre<T, N>(st + (p / 3) * RL + (p % 3), S + p * PL, tw, k);
+                c2r_pre<T, N>(st + (p / 3) * RL + (p % 3), S + p * PL, tw, k, kin);
             }
             __syncthreads();
             dif<T, M, true, NP, LP, 2, N, MRR>(S, tw, tid, ROW_THREADS);
@@ -1235,14 +1350,40 @@ row_nonlin(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __re
     if constexpr (WRITE_RU)
         for (int i = tid; i < M; i += RNL_THREADS) posn[i] = dif_position<M, MRR>(i);
 
+    // kx columns that the rows of a member hold on each side (read again only
+    // where the member changes)
+    int pm = -1, pc = M + 1;
+    auto cols = [&](int mm, int side) {
+        if constexpr (can_prune<T, N>()) {
+            if (mm != pm) {
+                pm = mm;
+                pc = mem[mm].kp.pcols;
+            }
+            return rl.prune & side ? pc : M + 1;
+        } else {
+            return M + 1;
+        }
+    };
     auto issue = [&](int tt) {
         const int mm = tt / tiles_per, tl = tt - mm * tiles_per;
         const cpx<T>* su = mbuf(mem[mm], rl.in0) + (size_t)tl * ROWS * RL;
         const cpx<T>* sw = mbuf(mem[mm], rl.in1) + (size_t)tl * ROWS * RL;
-        for (int e = tid; e < 2 * NV; e += RNL_THREADS) {
-            const int b = e >= NV ? 1 : 0;
-            const int v = e - b * NV;
-            cp_async16(&st[b * ROWS * RL + v * VPE], &(b ? sw : su)[v * VPE]);
+        const int kin = cols(mm, PRUNE_IN);
+        if (kin >= M) {
+            for (int e = tid; e < 2 * NV; e += RNL_THREADS) {
+                const int b = e >= NV ? 1 : 0;
+                const int v = e - b * NV;
+                cp_async16(&st[b * ROWS * RL + v * VPE], &(b ? sw : su)[v * VPE]);
+            }
+        } else {  // the rows' first kin columns, zeros after them
+            constexpr int RV = RL / VPE;
+            for (int e = tid; e < 2 * NV; e += RNL_THREADS) {
+                const int b = e >= NV ? 1 : 0;
+                const int v = e - b * NV;
+                cpx<T>* dst = &st[b * ROWS * RL + v * VPE];
+                if ((v % RV) * VPE < kin * 3) cp_async16(dst, &(b ? sw : su)[v * VPE]);
+                else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
         }
     };
     int t = blockIdx.x;
@@ -1253,6 +1394,7 @@ row_nonlin(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __re
         __syncthreads();
         const int m = t / tiles_per, tl = t - m * tiles_per;
         const size_t row0 = (size_t)tl * ROWS;
+        const int kin = cols(m, PRUNE_IN), kout = cols(m, PRUNE_OUT);
 
         // A: C2R pre-processing + DIF stage 0, staging rows -> pencils
         for (int e = tid; e < 6 * ROWS * H0; e += RNL_THREADS) {
@@ -1283,7 +1425,7 @@ row_nonlin(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __re
                 }
             } else {
                 // item 0: k = S0 q pairs with S0 (R0 - q); X[0] with X[M]
-                const T x0 = va[0].x, xm = x[3 * M].x;
+                const T x0 = va[0].x, xm = M < kin ? x[3 * M].x : (T)0;
                 va[0] = mk<T>(x0 + xm, x0 - xm);
 #pragma unroll
                 for (int q = 1; q < R0 / 2; ++q) {
@@ -1499,6 +1641,7 @@ row_nonlin(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __re
             float4* dst = reinterpret_cast<float4*>(wout);
             for (int v = tid; v < NV; v += RNL_THREADS) {
                 const int r = v / (RL / VPE);
+                if (kout < M && (v - r * (RL / VPE)) * VPE >= kout * 3) continue;
                 const cpx<T>* s = P + r * RG + (v - r * (RL / VPE)) * VPE;
                 float4 val;
                 if constexpr (VPE == 2) {

@@ -43,11 +43,11 @@ int Engine<T, N>::stats(bfg_ctx* c, int cfield, double max_est, int nbins, doubl
         d_spart, SPEC_BLOCKS, (int)spec_q, d_spec);
     if ((rc = after_launch(c, "spectrum_final"))) return rc;
     // real-space field into v2 (as [z][y][x][3] reals)
-    if ((rc = col<CM_IZ_PLAIN>(c, self(c), 1, roles(cfield, B_NONE, B_WB, B_NONE)))) return rc;
-    if ((rc = col<CM_Y_INV1>(c, self(c), 1, roles(B_WB, B_NONE, B_WB, B_NONE)))) return rc;
-    if ((rc = row<RM_C2R, false>(c, self(c), 1, roles(B_WB, B_NONE, B_NONE, B_NONE, B_NONE,
-                                                     B_NONE, B_NONE, B_V2))))
+    // (the velocity is zero outside kM, the state where it is known to be)
+    const int prune = cfield == B_WA || (cfield == B_W0 && !c->w0_full) ? PRUNE_IN : 0;
+    if ((rc = col<CM_IZ_PLAIN>(c, self(c), 1, pruned(roles(cfield, B_NONE, B_WB, B_NONE), prune))))
         return rc;
+    if ((rc = rspace(c, B_WB, B_V2, prune))) return rc;
     const double me3 = max_est * std::sqrt(3.0);
     const size_t npts = (size_t)N * N * N;
     CU(ensure_smem(moments_kernel<T>, (size_t)nbins * 4 * 4, c->device));

@@ -189,6 +189,17 @@ row_nonlin_warp(const Member<float>* __restrict__ mem, const Roles rl,
         const size_t r = (size_t)(row - m * rows_per);
         return mbuf(mem[m], b ? rl.in1 : rl.in0) + r * RL;
     };
+    // kx columns that the rows of a member hold on each side (read again only
+    // where the member changes)
+    int pm = -1, pc = M + 1;
+    auto cols = [&](int row, int side) {
+        const int m = row / rows_per;
+        if (m != pm) {
+            pm = m;
+            pc = mem[m].kp.pcols;
+        }
+        return rl.prune & side ? pc : M + 1;
+    };
     // loads are issued by lane 0 after every lane's earlier reads of the
     // destination (fence: ordered before the async proxy's writes) and after
     // the bulk stores that read it (wait_group.read)
@@ -198,8 +209,10 @@ row_nonlin_warp(const Member<float>* __restrict__ mem, const Roles rl,
         __syncwarp();
         if (lane == 0) {
             unsigned long long* bb = b ? bar_w : bar_u;
-            mbar_expect_tx(bb, ROW_BYTES);
-            bulk_load(b ? S.sw : S.su, row_src(row, b), ROW_BYTES, bb);
+            const int kc = cols(row, PRUNE_IN);
+            const unsigned bytes = kc < M ? kc * 3 * (unsigned)sizeof(C) : ROW_BYTES;
+            mbar_expect_tx(bb, bytes);
+            bulk_load(b ? S.sw : S.su, row_src(row, b), bytes, bb);
         }
     };
     if (gw < nrows) {
@@ -214,11 +227,19 @@ row_nonlin_warp(const Member<float>* __restrict__ mem, const Roles rl,
         const int m = row / rows_per;
         const size_t r = (size_t)(row - m * rows_per);
         const int next = row + nw;
+        const int kin = cols(row, PRUNE_IN), kout = cols(row, PRUNE_OUT);
         C U[3][8], Wv[3][8];
         // u: C2R pre-processing and inverse transforms (su -> U)
         ok = mbar_wait_bounded(bar_u, par_u);
         par_u ^= 1u;
         if (!ok) break;
+        // columns from kin on are zero
+        auto fill = [&](C* st) {
+            if (kin > M) return;
+            for (int e = 3 * kin + lane; e < 3 * (M + 1); e += 32) st[e] = zero_c<float>();
+            __syncwarp();
+        };
+        fill(S.su);
 #pragma unroll
         for (int f = 0; f < 6; ++f) {
             if (f == 3) {
@@ -250,6 +271,7 @@ row_nonlin_warp(const Member<float>* __restrict__ mem, const Roles rl,
                 ok = mbar_wait_bounded(bar_w, par_w);
                 par_w ^= 1u;
                 if (!ok) break;
+                fill(S.sw);
             }
             const C* st = f < 3 ? S.su : S.sw;
             const int c = f % 3;
@@ -318,7 +340,8 @@ row_nonlin_warp(const Member<float>* __restrict__ mem, const Roles rl,
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) {
-            bulk_store(mbuf(mem[m], rl.out0) + r * RL, S.sw, ROW_BYTES);
+            bulk_store(mbuf(mem[m], rl.out0) + r * RL, S.sw,
+                       kout < M ? kout * 3 * (unsigned)sizeof(C) : ROW_BYTES);
             bulk_commit();
         }
         // the next row's w once the store has read sw
@@ -557,14 +580,37 @@ row_nonlin_wg(const Member<float>* __restrict__ mem, const Roles rl,
         const size_t r = (size_t)(row0 - m * rows_per);
         return mbuf(mem[m], b ? rl.in1 : rl.in0) + r * RL;
     };
+    // kx columns that the rows of a block's member hold on each side (a block
+    // never straddles members; read again only where the member changes)
+    int pm = -1, pc = M + 1;
+    auto cols = [&](int blk, int side) {
+        if constexpr (can_prune<float, N>()) {
+            const int m = blk * Q / rows_per;
+            if (m != pm) {
+                pm = m;
+                pc = mem[m].kp.pcols;
+            }
+            return rl.prune & side ? pc : M + 1;
+        } else {
+            return M + 1;
+        }
+    };
     auto issue = [&](int blk, int b) {
         bulk_wait_read();
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) {
             unsigned long long* bb = b ? bar_w : bar_u;
-            mbar_expect_tx(bb, BLOCK_BYTES);
-            bulk_load(b ? S.sw : S.su, block_src(blk, b), BLOCK_BYTES, bb);
+            const int kc = cols(blk, PRUNE_IN);
+            if (kc < M) {  // the rows' first kc columns, one copy per row
+                const unsigned bytes = kc * 3 * (unsigned)sizeof(C);
+                mbar_expect_tx(bb, Q * bytes);
+                for (int q = 0; q < Q; ++q)
+                    bulk_load((b ? S.sw : S.su) + q * RL, block_src(blk, b) + q * RL, bytes, bb);
+            } else {
+                mbar_expect_tx(bb, BLOCK_BYTES);
+                bulk_load(b ? S.sw : S.su, block_src(blk, b), BLOCK_BYTES, bb);
+            }
         }
     };
     if (gw < nblk) {
@@ -578,10 +624,18 @@ row_nonlin_wg(const Member<float>* __restrict__ mem, const Roles rl,
         const int m = row0 / rows_per;
         const size_t r0 = (size_t)(row0 - m * rows_per);
         const int next = blk + nw;
+        const int kin = cols(blk, PRUNE_IN), kout = cols(blk, PRUNE_OUT);
         C U[3][8], Wv[3][8];
         ok = mbar_wait_bounded(bar_u, par_u);
         par_u ^= 1u;
         if (!ok) break;
+        // columns from kin on are zero
+        auto fill = [&](C* st) {
+            if (kin > M) return;
+            for (int e = 3 * kin + l; e < 3 * (M + 1); e += G) st[rr_ * RL + e] = zero_c<float>();
+            __syncwarp();
+        };
+        fill(S.su);
 #pragma unroll
         for (int f = 0; f < 6; ++f) {
             if (f == 3) {
@@ -609,6 +663,7 @@ row_nonlin_wg(const Member<float>* __restrict__ mem, const Roles rl,
                 ok = mbar_wait_bounded(bar_w, par_w);
                 par_w ^= 1u;
                 if (!ok) break;
+                fill(S.sw);
             }
             const C* st = (f < 3 ? S.su : S.sw) + rr_ * RL;
             const int c = f % 3;
@@ -675,7 +730,12 @@ row_nonlin_wg(const Member<float>* __restrict__ mem, const Roles rl,
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) {
-            bulk_store(mbuf(mem[m], rl.out0) + r0 * RL, S.sw, BLOCK_BYTES);
+            C* dst = mbuf(mem[m], rl.out0) + r0 * RL;
+            if (kout < M)
+                for (int q = 0; q < Q; ++q)
+                    bulk_store(dst + q * RL, S.sw + q * RL, kout * 3 * (unsigned)sizeof(C));
+            else
+                bulk_store(dst, S.sw, BLOCK_BYTES);
             bulk_commit();
         }
         if (next < nblk) issue(next, 1);

@@ -158,6 +158,17 @@ row_c2r_bulk(const Member<float>* __restrict__ mem, const Roles rl, float* __res
     Smem<N>* sp;
     const Warp<N> w = setup<N>(xr_smem, tw_g, nrows, &sp);
     Smem<N>& S = *sp;
+    // kx columns that the rows of a member hold (passes.cuh, modes outside kM)
+    int pm = -1, pc = M + 1;
+    auto cols = [&](int m) {
+        if constexpr (can_prune<float, N>()) {
+            if (m != pm) {
+                pm = m;
+                pc = rl.prune & PRUNE_IN ? mem[m].kp.pcols : M + 1;
+            }
+        }
+        return pc;
+    };
     auto issue = [&](int blk) {
         bulk_wait_read();
         fence_proxy_async();
@@ -165,8 +176,16 @@ row_c2r_bulk(const Member<float>* __restrict__ mem, const Roles rl, float* __res
         if (w.lane == 0) {
             const int m = blk * Q / rows_per;
             const size_t r = (size_t)(blk * Q - m * rows_per);
-            mbar_expect_tx(w.bar, IN_BYTES);
-            bulk_load(S.cr, mbuf(mem[m], rl.in0) + r * RL, IN_BYTES, w.bar);
+            const C* src = mbuf(mem[m], rl.in0) + r * RL;
+            const int kc = cols(m);
+            if (kc < M) {  // the rows' first kc columns, one copy per row
+                const unsigned bytes = kc * 3 * (unsigned)sizeof(C);
+                mbar_expect_tx(w.bar, Q * bytes);
+                for (int q = 0; q < Q; ++q) bulk_load(S.cr + q * RL, src + q * RL, bytes, w.bar);
+            } else {
+                mbar_expect_tx(w.bar, IN_BYTES);
+                bulk_load(S.cr, src, IN_BYTES, w.bar);
+            }
         }
     };
     if (w.first < w.nblk) issue(w.first);
@@ -177,7 +196,12 @@ row_c2r_bulk(const Member<float>* __restrict__ mem, const Roles rl, float* __res
         const int m = blk * Q / rows_per;
         const size_t r0 = (size_t)(blk * Q - m * rows_per);
         C V[3][8];
-        const C* st = S.cr + w.row * RL;
+        C* st = S.cr + w.row * RL;
+        const int kin = cols(m);
+        if (kin <= M) {  // columns from kin on are zero
+            for (int e = 3 * kin + w.l; e < 3 * (M + 1); e += G) st[e] = zero_c<float>();
+            __syncwarp();
+        }
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
 #pragma unroll

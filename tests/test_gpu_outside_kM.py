@@ -1,0 +1,130 @@
+"""The passes of a step leave out the modes outside kM (from 128^3 up): states
+that are zero there and states that are not, both dealiasing rules, boxes with
+unequal wavenumber spacings, stale values in every work buffer, ensembles of
+unequal members."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from oracle import nsve as O
+from bfps_b200 import _lib, ic
+from gpu_util import rel_err
+
+pytestmark = pytest.mark.gpu
+
+N = 128
+
+
+def _field(seed, dk, dealias, full):
+    """A random Hermitian field; zero outside kM unless `full`."""
+    rng = np.random.default_rng(seed)
+    w = O.dft(rng.standard_normal((N, N, N, 3))) / N ** 1.5
+    kk = O.KSpace(N, N, N, *dk, dealias)
+    w = w / (1.0 + kk.K2[..., None])
+    if not full:
+        w[kk.K2 >= kk.kM2] = 0
+    return O.symmetrize(w)
+
+
+def _solver(dk, dealias, precision="double"):
+    from bfps_b200.solver import vorticity_equation
+    ve = vorticity_equation(N, N, N, *dk, precision=precision, dealias_type=dealias)
+    ref = O.VorticityEquation(N, N, N, *dk, dealias_type=dealias, workers=8)
+    for o in (ve, ref):
+        o.nu, o.forcing_type, o.famplitude, o.fk0, o.fk1 = 0.02, "linear", 0.5, 1.5, 3.0
+    return ve, ref
+
+
+def _poison(ve):
+    """Large values in the work buffers and both RK buffers."""
+    L = _lib.lib()
+    big = np.full(ve.cshape, 1e6 * (1 + 1j), ve.cdtype)
+    spec = np.zeros((ve.kspace()["nshells"], 3, 3))
+    _lib.check(L.bfg_field_stats(ve.handle, big.ctypes.data_as(ctypes.c_void_p), 1.0, 16, _lib.ptr(spec),
+                                 None, None), ve.handle)
+    out = np.empty(ve.rshape, ve.rdtype)
+    _lib.check(L.bfg_ift(ve.handle, big.ctypes.data, out.ctypes.data), ve.handle)
+
+
+@pytest.mark.parametrize("dealias", [O.SMOOTH, O.TWO_THIRDS])
+@pytest.mark.parametrize("dk", [(1.0, 1.0, 1.0), (1.0, 0.5, 2.0), (0.7, 1.3, 1.0)])
+@pytest.mark.parametrize("full", [False, True])
+def test_step_matches_oracle(dealias, dk, full):
+    ve, ref = _solver(dk, dealias)
+    w0 = _field(3, dk, dealias, full)
+    ve.set_cvorticity(w0)
+    ref.cvorticity = w0.copy()
+    for s in range(2):
+        _poison(ve)
+        ve.step(1e-3)
+        ref.step(1e-3)
+        got = ve.get_cvorticity()
+        assert rel_err(got, ref.cvorticity) < 1e-12, s
+        # outside kM: exactly what the state held, or zero
+        out = ref.kk.K2 > ref.kk.kM2
+        assert (np.abs(got[out]).max() > 0) == full
+    st, want = ve.do_stats(2.0, 5.0, 32), O.nsve_do_stats(ref, 2.0, 5.0, 32)
+    for name in ("velocity", "vorticity"):
+        assert rel_err(st[name][0], want[name][0]) < 1e-12
+        assert rel_err(st[name][1], want[name][1]) < 1e-10
+    ve.velocity_rspace()
+    ur = ref.ift(ref.compute_velocity(ref.cvorticity))
+    assert rel_err(ve.get_rvelocity()[:, :, :N], ur) < 1e-12
+    ve.close()
+
+
+@pytest.mark.parametrize("dealias", [O.SMOOTH, O.TWO_THIRDS])
+def test_single_precision_and_replaced_states(dealias):
+    """Full state, then a zero-outside one, a checkpoint read of the full one
+    and a reset on one FP32 context."""
+    dk = (1.0, 1.0, 1.0)
+    ve, ref = _solver(dk, dealias, "single")
+    for full, read in ((True, False), (False, False), (True, True)):
+        w0 = _field(11, dk, dealias, full).astype(np.complex64)
+        _poison(ve)
+        if read:
+            ve.io_checkpoint_read(w0)
+            ref.cvorticity = ref.read_checkpoint_semantics(w0.astype(np.complex128))
+        else:
+            ve.set_cvorticity(w0)
+            ref.cvorticity = w0.astype(np.complex128)
+        ve.step(1e-3, 2)
+        ref.step(1e-3)
+        ref.step(1e-3)
+        assert rel_err(ve.get_cvorticity(), ref.cvorticity) < 2e-6, (full, read)
+    ve.reset()
+    ve.step(1e-3)
+    assert np.abs(ve.get_cvorticity()).max() == 0.0
+    ve.close()
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+def test_ensemble_of_unequal_members(precision):
+    """Members with different rules, boxes and states (one full, replaced while
+    in the ensemble): bit-identical to stepping alone."""
+    from bfps_b200.solver import ensemble
+    mk = [((1.0, 1.0, 1.0), O.SMOOTH, False), ((1.0, 1.0, 1.0), O.TWO_THIRDS, False),
+          ((1.0, 0.5, 2.0), O.SMOOTH, False)]
+    fields = [_field(20 + i, dk, de, fu) for i, (dk, de, fu) in enumerate(mk)]
+    replaced = _field(30, mk[1][0], mk[1][1], True)
+    alone, ens, members = [], ensemble(), []
+    for (dk, de, _), w in zip(mk, fields):
+        for group in (alone, members):
+            ve, _ = _solver(dk, de, precision)
+            ve.set_cvorticity(w)
+            group.append(ve)
+        ens.add(members[-1], 1e-3)
+    ens.step(2)
+    members[1].set_cvorticity(replaced)
+    ens.step(1)
+    for i, ve in enumerate(alone):
+        ve.step(1e-3, 2)
+        if i == 1:
+            ve.set_cvorticity(replaced)
+        ve.step(1e-3)
+    for a, b in zip(alone, members):
+        assert np.array_equal(a.get_cvorticity(), b.get_cvorticity())
+    ens.close()
+    for ve in alone + members:
+        ve.close()
