@@ -969,7 +969,8 @@ static int ensure_ru(bfg_ctx* c) {
 template <typename T, int NB, int MM>
 static int launch_tracers(bfg_ctx* c, const PParams& pp, bfg_pctx* p, double* out,
                           cudaStream_t st, const void* field) {
-    const unsigned blocks = (unsigned)((p->n + tracers_per_block<T>() - 1) / tracers_per_block<T>());
+    const int tpb = tracers_per_block<T>(pp.split);
+    const unsigned blocks = (unsigned)((p->n + tpb - 1) / tpb);
     if (blocks == 0) return 0;
     Prof pr(c, K_TRACER, st);
     tracer_kernel<T, NB, MM><<<blocks, TRACER_THREADS, 0, st>>>(
@@ -1007,6 +1008,8 @@ static PParams pparams(const bfg_pctx* p, double dt, int move) {
     pp.order = std::min(p->step_idx, p->nsteps);
     pp.accum = p->rhs0_zero ? 0 : 1;
     pp.move = move;
+    pp.split = c->real_bytes == 4 ? tracer_split<float>(p->n, p->neighbours)
+                                  : tracer_split<double>(p->n, p->neighbours);
     pp.dt = dt;
     return pp;
 }
@@ -2333,7 +2336,8 @@ static int ens_prepare(bfg_ens* e) {
         ts.pos = p->pos;
         ts.hist = p->hist;
         sets.push_back(ts);
-        const int64_t tpb = e->real_bytes == 4 ? tracers_per_block<float>() : tracers_per_block<double>();
+        const int64_t tpb = e->real_bytes == 4 ? tracers_per_block<float>(ts.pp.split)
+                                               : tracers_per_block<double>(ts.pp.split);
         start.push_back(start.back() + (p->n + tpb - 1) / tpb);
         e->batched.push_back(i);
     }

@@ -32,6 +32,7 @@ struct PParams {
     int order;        // AB order of this move
     int accum;        // rhs[0] += u(x) instead of =
     int move;         // 0: sample only (into out), 1: full loop
+    int split;        // lane groups of one tracer that share its z planes (tracer_split)
     double dt;
 };
 
@@ -64,104 +65,76 @@ __device__ __forceinline__ int wrap_once(int c, int N) {
     return c < 0 ? c + N : (c >= N ? c - N : c);
 }
 
-// x-segment of one stencil row: 2n+2 points x 3 components, contiguous in
-// [z][y][x][c] unless the stencil wraps across the periodic x boundary.
-// Loads 16-byte vectors from the aligned-down start and accumulates
-// sum_ix w[ix] * f(ix, c) in double.
-template <typename T, int NB>
-__device__ __forceinline__ void row_accumulate(const T* __restrict__ row, int x0, int N,
-                                               const double* wxc, double& a0, double& a1,
-                                               double& a2) {
-    constexpr int NP = 2 * NB + 2;
-    constexpr int VEC = 16 / (int)sizeof(T);  // elements per 16-byte vector
-    constexpr int NV = (3 * NP + VEC - 1) / VEC + 1;  // vectors covering any alignment
-    if (x0 >= 0 && x0 + NP <= N) {
-        const int e0 = x0 * 3;
-        const int base = e0 & ~(VEC - 1);
-        const int off = e0 - base;
-        T buf[NV * VEC];
-        const int maxv = (N * 3 - base) / VEC;  // vectors left in this row
-#pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            if (v < maxv) {
-                if constexpr (sizeof(T) == 4) {
-                    const float4 q = *reinterpret_cast<const float4*>(row + base + v * VEC);
-                    buf[v * 4 + 0] = q.x; buf[v * 4 + 1] = q.y;
-                    buf[v * 4 + 2] = q.z; buf[v * 4 + 3] = q.w;
-                } else {
-                    const double2 q = *reinterpret_cast<const double2*>(row + base + v * VEC);
-                    buf[v * 2 + 0] = q.x; buf[v * 2 + 1] = q.y;
-                }
-            } else {
-#pragma unroll
-                for (int u = 0; u < VEC; ++u) buf[v * VEC + u] = (T)0;
-            }
-        }
-#pragma unroll
-        for (int ix = 0; ix < NP; ++ix) {
-            T f[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const int j = ix * 3 + c;
-                // buf[j + off], off in [0, VEC)
-                T v = buf[j];
-#pragma unroll
-                for (int o = 1; o < VEC; ++o) v = (off == o) ? buf[j + o] : v;
-                f[c] = v;
-            }
-            a0 += (double)f[0] * wxc[ix];
-            a1 += (double)f[1] * wxc[ix];
-            a2 += (double)f[2] * wxc[ix];
-        }
-    } else {
-#pragma unroll
-        for (int ix = 0; ix < NP; ++ix) {
-            const int xx = wrap_once(x0 + ix, N);
-            a0 += (double)row[xx * 3 + 0] * wxc[ix];
-            a1 += (double)row[xx * 3 + 1] * wxc[ix];
-            a2 += (double)row[xx * 3 + 2] * wxc[ix];
-        }
-    }
-}
-
 // 32-byte vector load (one L1 sector per lane), sm_100; p 32-byte aligned
-__device__ __forceinline__ void ld_v8(const float* p, float* v) {
+__device__ __forceinline__ void ld_32b(const float* p, float* v) {
     asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]),
                    "=f"(v[6]), "=f"(v[7])
                  : "l"(p));
 }
+__device__ __forceinline__ void ld_32b(const double* p, double* v) {  // four doubles
+    asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
+                 : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+                 : "l"(p));
+}
 
 constexpr int TRACER_THREADS = 128;
 
-// Lanes that share one tracer: two for FP32 fields, one for FP64 fields.  A
-// stencil row is read as up to four (six for n = 5) 32-byte sectors from its
-// aligned-down start.  With one lane per tracer the gather is bound by L1
-// wavefronts (about one per sector, as each lane's sector lies in another
-// line); with the sectors of a row spread over two lanes of one load, a
-// wavefront serves both, and the per-row address and FP64 work only doubles.
-// Measured on B200 (4e6 tracers, n = 3, m = 2, 512^3): 3.26 ms with one lane,
-// 2.70 ms with two, 4.47 ms with four (issue bound).
+// Lanes that share one stencil row: two for FP32 fields, four for FP64 fields.
+// A row is read as 32-byte sectors from its aligned-down start (up to four in
+// FP32, nine in FP64 for n = 4).  With one lane per tracer the gather is bound
+// by L1 wavefronts (about one per sector, as each lane's sector lies in another
+// line); with the sectors of a row spread over the lanes of one load, a
+// wavefront serves them all, and only the per-row address and FP64 work grows.
+// Measured on B200, FP32 (4e6 tracers, n = 3, m = 2, 512^3): 3.26 ms with one
+// lane, 2.70 ms with two, 4.47 ms with four (issue bound).  FP64 (50001
+// tracers, n = 4, m = 1, 256^3): 490 us with one lane, 250 us with four (190 us
+// with the loop shape below).
 template <typename T>
 __host__ __device__ constexpr int tracer_lanes() {
-    return sizeof(T) == 4 ? 2 : 1;
+    return sizeof(T) == 4 ? 2 : 4;
 }
-// n = 3 stencils (8 rows per plane): the y loop of the FP32 gather is
-// unrolled, so the y weights stay in registers instead of local memory, and
-// the kernel is given the registers of five blocks per SM instead of six.
-// Measured on B200 (4e6 tracers, n = 3, m = 2): 2.57 against 2.70 ms at
-// 512^3; for n = 2 (ensembles) it was slower, for n = 4, 5 it spills.
-template <int NB>
-__host__ __device__ constexpr int tracer_row_unroll() {
-    return NB == 3 ? 2 * NB + 2 : 1;
-}
-template <int NB>
-__host__ __device__ constexpr int tracer_min_blocks() {
-    return NB == 3 ? 5 : 6;
+// Few tracers leave the chip waiting for one dependent row after another: then
+// up to eight lane groups share a tracer, group g taking the z planes g, g +
+// split, ..., as long as all groups together are no more than 256 threads per
+// SM (the gather of more threads is bound by throughput, and every group
+// repeats the cell and weight arithmetic).  It depends on the number of tracers
+// only, so a system sums in the same order alone and in an ensemble.  The FP32
+// n = 3 gather, unrolled up to its register limit, is not split (the runtime
+// plane stride spilled there: 2.47 -> 2.55 ms for 4e6 tracers).
+// 1024 tracers, FP64, n = 2: 45 us with one lane per tracer, 14 us with
+// four lanes a row and up to eight groups.
+template <typename T>
+__host__ __device__ constexpr bool tracer_splits(int nb) {
+    return sizeof(T) == 8 || nb != 3;
 }
 template <typename T>
-__host__ __device__ constexpr int tracers_per_block() {
-    return TRACER_THREADS / tracer_lanes<T>();
+__host__ __device__ inline int tracer_split(int64_t n, int nb) {
+    const int lanes = tracer_lanes<T>(), planes = 2 * nb + 2;
+    int r = 1;
+    if (!tracer_splits<T>(nb)) return r;
+    while (r < 8 && 2 * r <= planes && 2 * r * lanes <= 32 && n * lanes * 2 * r <= 148 * 256) r *= 2;
+    return r;
+}
+// The gather waits for its rows (long scoreboard): rows of the y loop are
+// unrolled so that several are in flight, and the kernels are given the
+// registers for that.  FP32: n = 3 its eight rows, four blocks per SM (4e6
+// tracers, 512^3: 2.43 ms; five blocks 2.47-2.52, four rows and six blocks 2.57);
+// the others three rows, four blocks (1e5 tracers, n = 2, m = 2, 256^3: 75 us;
+// one row and six blocks 100, two rows and five 94; six rows 76).  FP64: two
+// rows, three blocks (50001 tracers, n = 4, m = 1, 256^3: 190 us; one row and
+// four blocks 251, three rows 263, four rows and two blocks 217).
+template <typename T, int NB>
+__host__ __device__ constexpr int tracer_row_unroll() {
+    return sizeof(T) == 4 ? (NB == 3 ? 2 * NB + 2 : 3) : 2;
+}
+template <typename T, int NB>
+__host__ __device__ constexpr int tracer_min_blocks() {
+    return sizeof(T) == 8 ? 3 : 4;
+}
+template <typename T>
+__host__ __device__ inline int tracers_per_block(int split) {
+    return TRACER_THREADS / (tracer_lanes<T>() * split);
 }
 
 // sum of v over the L lanes of a tracer group, pairwise ((l0 + l1) + (l2 +
@@ -174,25 +147,27 @@ __device__ __forceinline__ double group_sum(double v, unsigned gmask) {
     return v;
 }
 
-// FP32 field (precision form), lane j (0..L-1) of the tracer's group, which
-// reads vectors j, j + L, ... of each row: the x sums of the stencil rows run
-// in FP32 with the x weights rounded to FP32, over the words a lane reads; the
-// y/z weights, the accumulation of those sums over the rows, the sum over the
-// lanes and everything after stay FP64.  Word i of the row segment read from the
+// Lane j (0..L-1) of a lane group reads vectors j, j + L, ... of each row of
+// the group's z planes (iz = z0, z0 + zs, ...).  FP32 field (precision form):
+// the x sums of the stencil rows run in FP32 with the x weights rounded to
+// FP32, over the words a lane reads; the y/z weights, the accumulation of those
+// sums over the rows, the sum over the lanes and everything after stay FP64.
+// FP64 field: all of it in FP64.  Word i of the row segment read from the
 // aligned-down start belongs to point (i - off) / 3, component
 // (i - off) mod 3, so each lane's x weights are shifted once per tracer and its
 // sums are kept per word phase i mod 3, mapped to components at the end.
 #ifndef BFG_TRACER_ROWSUM_F64
 #define BFG_TRACER_ROWSUM_F64 0
 #endif
-template <int NB, int L>
-__device__ __forceinline__ void row_gather_f32(const float* __restrict__ ru, int N, const int* g,
-                                               int x0, const double* wx, const double* wy,
-                                               const double* wz, int j, unsigned gmask,
-                                               double& a0, double& a1, double& a2) {
-    using SumT = typename std::conditional<BFG_TRACER_ROWSUM_F64 != 0, double, float>::type;
+template <typename T, int NB, int L>
+__device__ __forceinline__ void row_gather(const T* __restrict__ ru, int N, const int* g, int x0,
+                                           const double* wx, const double* wy, const double* wz,
+                                           int j, int z0, int zs, unsigned gmask, double& a0,
+                                           double& a1, double& a2) {
+    using SumT =
+        typename std::conditional<sizeof(T) == 8 || BFG_TRACER_ROWSUM_F64 != 0, double, float>::type;
     constexpr int NP = 2 * NB + 2;
-    constexpr int VW = 8;                                // floats per vector
+    constexpr int VW = 32 / (int)sizeof(T);              // values per vector
     constexpr int NVMAX = (3 * NP + 2 * (VW - 1)) / VW;  // vectors covering any alignment
     constexpr int VPL = (NVMAX + L - 1) / L;             // vectors per lane
     const size_t rowN = (size_t)N;
@@ -216,36 +191,37 @@ __device__ __forceinline__ void row_gather_f32(const float* __restrict__ ru, int
                 for (int pt = 0; pt < NP; ++pt) w = (k >= 3 * pt && k < 3 * pt + 3) ? wxf[pt] : w;
                 wl[t][u] = w;
             }
-        // word u of vector v = j + L t has phase (8 v + u) mod 3, that is
-        // (2 j + 2 L t + u) mod 3: the sums are kept per lane-relative phase
-        // (2 L t + u) mod 3 and rotated by 2 j at the end
+        // word u of vector v = j + L t has phase (VW v + u) mod 3: the sums are
+        // kept per lane-relative phase (VW L t + u) mod 3 and rotated by VW j
+        // at the end
         double ph[3] = {0.0, 0.0, 0.0};
 #pragma unroll 1
-        for (int iz = 0; iz < NP; ++iz) {
+        for (int iz = z0; iz < NP; iz += zs) {
             const int z = wrap_once(g[2] - NB + iz, N);
             const double bz = wz[iz];
-#pragma unroll(tracer_row_unroll<NB>())
+#pragma unroll(tracer_row_unroll<T, NB>())
             for (int iy = 0; iy < NP; ++iy) {
                 const int y = wrap_once(g[1] - NB + iy, N);
-                const float* row = ru + ((size_t)z * rowN + y) * rowN * 3 + base;
+                const T* row = ru + ((size_t)z * rowN + y) * rowN * 3 + base;
                 const double bzy = bz * wy[iy];
                 SumT sp[3] = {0, 0, 0};
 #pragma unroll
                 for (int t = 0; t < VPL; ++t) {
                     if (j + L * t < nv) {
-                        float q[VW];
-                        ld_v8(row + VW * (j + L * t), q);
+                        T q[VW];
+                        ld_32b(row + VW * (j + L * t), q);
 #pragma unroll
                         for (int u = 0; u < VW; ++u)
-                            sp[(2 * L * t + u) % 3] = fma((SumT)q[u], wl[t][u], sp[(2 * L * t + u) % 3]);
+                            sp[(VW * L * t + u) % 3] =
+                                fma((SumT)q[u], wl[t][u], sp[(VW * L * t + u) % 3]);
                     }
                 }
 #pragma unroll
                 for (int c = 0; c < 3; ++c) ph[c] = fma(bzy, (double)sp[c], ph[c]);
             }
         }
-        // lane-relative phase (k - 2 j) mod 3 holds phase k
-        const int r = (2 * j) % 3;
+        // lane-relative phase (k - VW j) mod 3 holds phase k
+        const int r = (VW * j) % 3;
         double G[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k)
@@ -272,13 +248,13 @@ __device__ __forceinline__ void row_gather_f32(const float* __restrict__ ru, int
         }
         double A[3] = {0.0, 0.0, 0.0};
 #pragma unroll 1
-        for (int iz = 0; iz < NP; ++iz) {
+        for (int iz = z0; iz < NP; iz += zs) {
             const int z = wrap_once(g[2] - NB + iz, N);
             const double bz = wz[iz];
-#pragma unroll(tracer_row_unroll<NB>())
+#pragma unroll(tracer_row_unroll<T, NB>())
             for (int iy = 0; iy < NP; ++iy) {
                 const int y = wrap_once(g[1] - NB + iy, N);
-                const float* row = ru + ((size_t)z * rowN + y) * rowN * 3;
+                const T* row = ru + ((size_t)z * rowN + y) * rowN * 3;
                 SumT s0 = 0, s1 = 0, s2 = 0;
 #pragma unroll
                 for (int m = 0; m < PPL; ++m) {
@@ -300,13 +276,13 @@ __device__ __forceinline__ void row_gather_f32(const float* __restrict__ ru, int
     }
 }
 
-// tracer i of one system, lane j of its group (tracer_lanes<T>() lanes; gmask
-// the group's lanes): gather u(x_i), then (move) the Adams-Bashforth step.
-// With four lanes, lane d < 3 finishes component d.
+// tracer i of one system, lane `sub` of its pp.split groups of
+// tracer_lanes<T>() lanes (gmask: all of them): gather u(x_i), then (move) the
+// Adams-Bashforth step, whose components the first lanes finish.
 template <typename T, int NB, int MM>
 __device__ __forceinline__ void tracer_one(const PParams& pp, const T* __restrict__ ru,
                                            double* __restrict__ pos, double* __restrict__ hist,
-                                           double* __restrict__ sample_out, int64_t i, int j,
+                                           double* __restrict__ sample_out, int64_t i, int sub,
                                            unsigned gmask) {
     constexpr int NP = 2 * NB + 2;
     constexpr int L = tracer_lanes<T>();
@@ -324,28 +300,15 @@ __device__ __forceinline__ void tracer_one(const PParams& pp, const T* __restric
     beta_weights<NB, MM>(fr[2], wz);
 
     double acc[3] = {0.0, 0.0, 0.0};
-    const size_t rowN = (size_t)N;
-    const int x0 = g[0] - NB;
-    if constexpr (sizeof(T) == 4) {
-        row_gather_f32<NB, L>(reinterpret_cast<const float*>(ru), N, g, x0, wx, wy, wz, j, gmask,
-                           acc[0], acc[1], acc[2]);
-    } else {
-#pragma unroll 1
-        for (int iz = 0; iz < NP; ++iz) {
-            const int z = wrap_once(g[2] - NB + iz, N);
-#pragma unroll 1
-            for (int iy = 0; iy < NP; ++iy) {
-                const int y = wrap_once(g[1] - NB + iy, N);
-                // coefficient (bz * by) * bx of apply_computation
-                const double bzy = wz[iz] * wy[iy];
-                double wxc[NP];
+    const int z0 = tracer_splits<T>(NB) ? sub / L : 0, zs = tracer_splits<T>(NB) ? pp.split : 1;
+    row_gather<T, NB, L>(ru, N, g, g[0] - NB, wx, wy, wz, sub % L, z0, zs, gmask, acc[0], acc[1],
+                         acc[2]);
+    // the groups' planes, pairwise; every lane of the tracer gets the sum
+    for (int o = L; o < L * zs; o *= 2)
 #pragma unroll
-                for (int ix = 0; ix < NP; ++ix) wxc[ix] = bzy * wx[ix];
-                row_accumulate<T, NB>(ru + ((size_t)z * rowN + y) * rowN * 3, x0, N, wxc, acc[0],
-                                      acc[1], acc[2]);
-            }
-        }
-    }
+        for (int d = 0; d < 3; ++d) acc[d] += __shfl_xor_sync(gmask, acc[d], o);
+    const int j = sub;  // lane j < L finishes components j, j + L, ...
+    if (j >= L) return;
     if (!pp.move) {
 #pragma unroll
         for (int d = 0; d < 3; ++d)
@@ -394,22 +357,26 @@ __device__ __forceinline__ void tracer_one(const PParams& pp, const T* __restric
     }
 }
 
-// lanes of the calling thread's tracer group, as a shuffle mask
-template <int L>
-__device__ __forceinline__ unsigned tracer_group_mask() {
+// lanes of one tracer (a power of two)
+template <typename T, int NB>
+__device__ __forceinline__ int tracer_lanes_of(const PParams& pp) {
+    return tracer_splits<T>(NB) ? tracer_lanes<T>() * pp.split : tracer_lanes<T>();
+}
+// lanes of the calling thread's tracer (LR of them), as a shuffle mask
+__device__ __forceinline__ unsigned tracer_group_mask(int LR) {
     const int lane = threadIdx.x & 31;
-    return L == 1 ? (1u << lane) : (((1u << L) - 1u) << (lane & ~(L - 1)));
+    return (LR == 32 ? 0xffffffffu : (1u << LR) - 1u) << (lane & ~(LR - 1));
 }
 
 template <typename T, int NB, int MM>
-__global__ void __launch_bounds__(TRACER_THREADS, tracer_min_blocks<NB>())
+__global__ void __launch_bounds__(TRACER_THREADS, tracer_min_blocks<T, NB>())
 tracer_kernel(const PParams pp, const T* __restrict__ ru, double* __restrict__ pos,
               double* __restrict__ hist, double* __restrict__ sample_out) {
-    constexpr int L = tracer_lanes<T>();
+    const int LR = tracer_lanes_of<T, NB>(pp);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t i = t / L;
-    if (i >= pp.n) return;  // whole groups leave together
-    tracer_one<T, NB, MM>(pp, ru, pos, hist, sample_out, i, (int)(t % L), tracer_group_mask<L>());
+    const int64_t i = t >> (__ffs(LR) - 1);
+    if (i >= pp.n) return;  // all lanes of a tracer leave together
+    tracer_one<T, NB, MM>(pp, ru, pos, hist, sample_out, i, (int)t & (LR - 1), tracer_group_mask(LR));
 }
 
 // the tracer systems of many ensemble members in one launch
@@ -436,7 +403,7 @@ __global__ void tracer_sets_advance(TracerSet* __restrict__ sets, int nsets) {
 // bstart[k] <= b < bstart[k+1]; the set is found once per block and its
 // descriptor copied to shared memory.
 template <typename T, int NB, int MM>
-__global__ void __launch_bounds__(TRACER_THREADS, tracer_min_blocks<NB>())
+__global__ void __launch_bounds__(TRACER_THREADS, tracer_min_blocks<T, NB>())
 tracer_batch_kernel(const TracerSet* __restrict__ sets, const int64_t* __restrict__ bstart,
                     int nsets) {
     __shared__ TracerSet s;
@@ -459,11 +426,12 @@ tracer_batch_kernel(const TracerSet* __restrict__ sets, const int64_t* __restric
         for (int w = threadIdx.x; w < (int)(sizeof(TracerSet) / 4); w += blockDim.x) dst[w] = src[w];
     }
     __syncthreads();
-    constexpr int L = tracer_lanes<T>();
-    const int64_t i = ((int64_t)blockIdx.x - bstart[s_k]) * (blockDim.x / L) + threadIdx.x / L;
-    if (i >= s.pp.n) return;  // whole groups leave together
-    tracer_one<T, NB, MM>(s.pp, (const T*)s.ru, s.pos, s.hist, nullptr, i, (int)(threadIdx.x % L),
-                          tracer_group_mask<L>());
+    const int LR = tracer_lanes_of<T, NB>(s.pp);
+    const int64_t t = ((int64_t)blockIdx.x - bstart[s_k]) * blockDim.x + threadIdx.x;
+    const int64_t i = t >> (__ffs(LR) - 1);
+    if (i >= s.pp.n) return;  // all lanes of a tracer leave together
+    tracer_one<T, NB, MM>(s.pp, (const T*)s.ru, s.pos, s.hist, nullptr, i, (int)t & (LR - 1),
+                          tracer_group_mask(LR));
 }
 
 // ---------------------------------------------------------------------------
