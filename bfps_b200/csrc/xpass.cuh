@@ -12,10 +12,10 @@
 //     row as soon as this row's output has left, so both arrive while the
 //     warp still computes;
 //   * a 256-point transform lives in registers, eight values per lane:
-//     one radix-8 butterfly over registers, then two exchanges through the
-//     warp's own shared buffer (radix-8 over 8-lane groups, radix-4 over
-//     4-lane groups), so no step of a row waits for another warp
-//     (__syncwarp only, no block barrier);
+//     one radix-8 butterfly over registers, an exchange through the warp's
+//     own shared buffer (radix-8 over 8-lane groups) and one by shuffles
+//     (radix-4 over 4-lane groups), so no step of a row waits for another
+//     warp (__syncwarp only, no block barrier);
 //   * the product is formed in registers on the transformed values of all
 //     six transforms (every transform leaves the grid points in the same
 //     lane / register order);
@@ -29,9 +29,18 @@
 // k = l + 32 q: W_256^{nk} = W_256^{n1 l} W_8^{n1 q} W_32^{n2 l}, and the
 // 32-point factor splits again with n2 = m1 + 8 m2, l = l1 + 4 l2.
 //
-// Shared-memory pitches keep every exchange free of bank conflicts for
-// 8-byte accesses (half-warp wavefronts): [n1][l] rows of 36, [n1][l1][m1]
-// blocks of 68 / 17.
+// The exchange pitch keeps it free of bank conflicts for 8-byte accesses
+// (half-warp wavefronts): [n1][l] rows of 36.
+//
+// Bound by the shared-memory data pipe (79 % of its wavefronts at 256^3 when
+// both exchanges went through it and every transform read its twiddles there),
+// not by DRAM: so the last exchange is made of shuffles of half the values (16
+// wavefronts instead of 32 for radix 4, 8 for the radix 2 below), and the
+// twiddles W_M^{n1 l}, the same for all nine transforms of a row, stay in
+// registers; the forward transform applies them after its exchange, where they
+// are the lane's own; the mirror values of the R2C post-processing come by
+// shuffles too (16 wavefronts instead of 32).  256^3: 197 -> 173 us, 512^3: 1480 ->
+// 1390 us per launch.
 #pragma once
 #include "bulk.cuh"
 #include "passes.cuh"
@@ -42,9 +51,7 @@ namespace xw {
 
 constexpr int NWARP = 12;              // warps per CTA, one CTA per SM
 constexpr int XP1 = 36;                // exchange [n1][l] row pitch
-constexpr int XP2 = 68, XQ2 = 17;      // exchange [n1][l1][m1] pitches
-constexpr int XBUF = 8 * XP2;          // 544 >= 8 * XP1, >= 256
-constexpr int T1P = 36;                // twiddle table [n1][l] row pitch
+constexpr int XBUF = 8 * XP1;          // 288 >= 256
 constexpr int T2P = 9;                 // twiddle table [l1][m1] row pitch: the inverse
                                        // reads it with l1 over the lanes, which a
                                        // pitch of 8 puts on two banks for four rows
@@ -57,13 +64,47 @@ struct Smem {
     cpx<float> x[XBUF];                         // exchanges
 };
 
-// 256-point inverse transform (sign +): Z[l + 32 q] in v[q] -> grid order
+__device__ __forceinline__ cpx<float> shfl_c(cpx<float> v, int m) {
+    return mk<float>(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
+}
+__device__ __forceinline__ cpx<float> pick(bool c, cpx<float> a, cpx<float> b) {
+    return mk<float>(c ? a.x : b.x, c ? a.y : b.y);
+}
+// Z[M - k] for k = l + G q of a spectrum Z[l + G q] in v[q] over G lanes: register
+// 7 - q of lane G - l, or of lane 0 (l = 0) register 8 - q; the value for k = 0
+// is not used
+template <int G>
+__device__ __forceinline__ cpx<float> mirror(const cpx<float> (&v)[8], int q, int l) {
+    const int src = l == 0 ? 0 : G - l;
+    const cpx<float> o = mk<float>(__shfl_sync(0xffffffffu, v[7 - q].x, src, G),
+                                   __shfl_sync(0xffffffffu, v[7 - q].y, src, G));
+    return pick(l == 0, v[(8 - q) & 7], o);
+}
+// 4 x 4 transpose over the four lanes j of a group: lane j's r[i] becomes lane
+// i's r[j] (two exchanges of half the values, no shared memory)
+__device__ __forceinline__ void transpose4(cpx<float>* r, int j) {
+#pragma unroll
+    for (int m = 1; m <= 2; m *= 2) {
+        const bool up = (j & m) != 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (i & m) continue;
+            // the lower lane keeps r[i] and gives r[i + m], the upper the reverse
+            const cpx<float> got = shfl_c(pick(up, r[i], r[i + m]), m);
+            r[i] = pick(up, got, r[i]);
+            r[i + m] = pick(up, r[i + m], got);
+        }
+    }
+}
+
+// 256-point inverse transform (sign +): Z[l + 32 q] in v[q] -> grid order;
+// t1r[n1] = W_256^{n1 l} of this lane
 __device__ __forceinline__ void inv256(cpx<float> (&v)[8], cpx<float>* xb,
-                                       const cpx<float>* __restrict__ t1,
+                                       const cpx<float> (&t1r)[8],
                                        const cpx<float>* __restrict__ t2, int lane) {
     dft<float, true, 8>(v);  // over q -> n1
 #pragma unroll
-    for (int n1 = 1; n1 < 8; ++n1) v[n1] = cmulc(v[n1], t1[n1 * T1P + lane]);  // W_256^{-n1 l}
+    for (int n1 = 1; n1 < 8; ++n1) v[n1] = cmulc(v[n1], t1r[n1]);  // W_256^{-n1 l}
     __syncwarp();
 #pragma unroll
     for (int n1 = 0; n1 < 8; ++n1) xb[n1 * XP1 + lane] = v[n1];
@@ -74,63 +115,37 @@ __device__ __forceinline__ void inv256(cpx<float> (&v)[8], cpx<float>* xb,
     dft<float, true, 8>(v);  // over l2 -> m1
 #pragma unroll
     for (int m1 = 1; m1 < 8; ++m1) v[m1] = cmulc(v[m1], t2[l1 * T2P + m1]);  // W_32^{-l1 m1}
-    __syncwarp();
-#pragma unroll
-    for (int m1 = 0; m1 < 8; ++m1) xb[n1 * XP2 + l1 * XQ2 + m1] = v[m1];
-    __syncwarp();
-    const int j = lane & 3;
-    cpx<float> a[4], b[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        a[i] = xb[n1 * XP2 + i * XQ2 + j];
-        b[i] = xb[n1 * XP2 + i * XQ2 + j + 4];
-    }
-    dft<float, true, 4>(a);  // over l1 -> m2
-    dft<float, true, 4>(b);
-#pragma unroll
-    for (int m2 = 0; m2 < 4; ++m2) {
-        v[m2] = a[m2];
-        v[4 + m2] = b[m2];
-    }
+    // lane j of the group takes m1 = j and j + 4 of every l1
+    transpose4(v, l1);
+    transpose4(v + 4, l1);
+    dft<float, true, 4>(v);  // over l1 -> m2
+    dft<float, true, 4>(v + 4);
 }
 
 // 256-point forward transform (sign -): grid order in -> Z[l + 32 q] in v[q]
 __device__ __forceinline__ void fwd256(cpx<float> (&v)[8], cpx<float>* xb,
-                                       const cpx<float>* __restrict__ t1,
+                                       const cpx<float> (&t1r)[8],
                                        const cpx<float>* __restrict__ t2, int lane) {
     const int n1 = lane >> 2, j = lane & 3;
-    cpx<float> a[4], b[4];
-#pragma unroll
-    for (int m2 = 0; m2 < 4; ++m2) {
-        a[m2] = v[m2];
-        b[m2] = v[4 + m2];
-    }
-    dft<float, false, 4>(a);  // over m2 -> l1
-    dft<float, false, 4>(b);
+    dft<float, false, 4>(v);  // over m2 -> l1
+    dft<float, false, 4>(v + 4);
 #pragma unroll
     for (int l1 = 1; l1 < 4; ++l1) {
-        a[l1] = cmul(a[l1], t2[l1 * T2P + j]);      // W_32^{m1 l1}, m1 = j
-        b[l1] = cmul(b[l1], t2[l1 * T2P + j + 4]);  // m1 = j + 4
+        v[l1] = cmul(v[l1], t2[l1 * T2P + j]);              // W_32^{m1 l1}, m1 = j
+        v[4 + l1] = cmul(v[4 + l1], t2[l1 * T2P + j + 4]);  // m1 = j + 4
     }
-    __syncwarp();
-#pragma unroll
-    for (int l1 = 0; l1 < 4; ++l1) {
-        xb[n1 * XP2 + l1 * XQ2 + j] = a[l1];
-        xb[n1 * XP2 + l1 * XQ2 + j + 4] = b[l1];
-    }
-    __syncwarp();
-    const int l1 = lane & 3;
-#pragma unroll
-    for (int m1 = 0; m1 < 8; ++m1) v[m1] = xb[n1 * XP2 + l1 * XQ2 + m1];
+    // lane l1 of the group takes every m1
+    transpose4(v, j);
+    transpose4(v + 4, j);
+    const int l1 = j;
     dft<float, false, 8>(v);  // over m1 -> l2
-#pragma unroll
-    for (int l2 = 0; l2 < 8; ++l2) v[l2] = cmul(v[l2], t1[n1 * T1P + l1 + 4 * l2]);  // W_256^{n1 l}
     __syncwarp();
 #pragma unroll
     for (int l2 = 0; l2 < 8; ++l2) xb[n1 * XP1 + l1 + 4 * l2] = v[l2];
     __syncwarp();
+    v[0] = xb[lane];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = xb[i * XP1 + lane];
+    for (int i = 1; i < 8; ++i) v[i] = cmul(xb[i * XP1 + lane], t1r[i]);  // W_256^{n1 l}
     dft<float, false, 8>(v);  // over n1 -> q
 }
 
@@ -142,7 +157,7 @@ __device__ __forceinline__ void fwd256(cpx<float> (&v)[8], cpx<float>* xb,
 template <int N>
 __host__ __device__ constexpr size_t xw_smem_bytes() {
     return (size_t)xw::NWARP * sizeof(xw::Smem<N>) +
-           (size_t)(N + 8 * xw::T1P + 4 * xw::T2P) * sizeof(cpx<float>) + xw::NWARP * 16;
+           (size_t)(N + 4 * xw::T2P) * sizeof(cpx<float>) + xw::NWARP * 16;
 }
 
 template <int N, bool WRITE_RU>
@@ -162,16 +177,14 @@ row_nonlin_warp(const Member<float>* __restrict__ mem, const Roles rl,
     extern __shared__ __align__(128) unsigned char xw_smem_raw[];
     Smem<N>* ws = reinterpret_cast<Smem<N>*>(xw_smem_raw);
     C* tw = reinterpret_cast<C*>(ws + NWARP);  // exp(-2 pi i m / N), m < N
-    C* t1 = tw + N;                            // [n1][l] = W_256^{n1 l}, pitch 36
-    C* t2 = t1 + 8 * T1P;                      // [l1][m1] = W_32^{l1 m1}, pitch T2P
+    C* t2 = tw + N;                            // [l1][m1] = W_32^{l1 m1}, pitch T2P
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(t2 + 4 * T2P);
 
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (int i = tid; i < N; i += blockDim.x) tw[i] = tw_g[i];
-    for (int i = tid; i < 8 * 32; i += blockDim.x) {
-        const int n1 = i >> 5, l = i & 31;
-        t1[n1 * T1P + l] = tw_g[(2 * n1 * l) % N];
-    }
+    C t1r[8];  // W_256^{n1 l} of this lane
+#pragma unroll
+    for (int n1 = 0; n1 < 8; ++n1) t1r[n1] = tw_g[(2 * n1 * lane) % N];
     if (tid < 32) t2[(tid >> 3) * T2P + (tid & 7)] = tw_g[16 * ((tid >> 3) * (tid & 7))];
     if (tid < 2 * NWARP) mbar_init(&bars[tid], 1);
     fence_mbar_init();
@@ -287,7 +300,7 @@ row_nonlin_warp(const Member<float>* __restrict__ mem, const Roles rl,
                     v[q] = c2r_lo(a, st[3 * (M - k) + c], tw[k]);
                 }
             }
-            xw::inv256(v, S.x, t1, t2, lane);
+            xw::inv256(v, S.x, t1r, t2, lane);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 if (f < 3) U[c][i] = v[i];
@@ -318,20 +331,17 @@ row_nonlin_warp(const Member<float>* __restrict__ mem, const Roles rl,
             C v[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = U[c][i];
-            xw::fwd256(v, S.x, t1, t2, lane);
-            __syncwarp();
-#pragma unroll
-            for (int q = 0; q < 8; ++q) S.x[lane + 32 * q] = v[q];  // natural order
-            __syncwarp();
+            xw::fwd256(v, S.x, t1r, t2, lane);
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const int k = lane + 32 * q;
+                const C zm = xw::mirror<32>(v, q, lane);
                 if (k == 0) {
                     const C z0 = v[0];
                     S.sw[c] = mk<float>(z0.x + z0.y, 0.f);
                     S.sw[3 * M + c] = mk<float>(z0.x - z0.y, 0.f);
                 } else {
-                    S.sw[3 * k + c] = r2c_lo(v[q], S.x[M - k], tw[k]);
+                    S.sw[3 * k + c] = r2c_lo(v[q], zm, tw[k]);
                 }
             }
         }
@@ -362,8 +372,7 @@ row_nonlin_warp(const Member<float>* __restrict__ mem, const Roles rl,
 //           l + 4: two radix-4 over l;
 //   G = 8:  one exchange [n1][l] (pitch 9), radix 8 over l;
 //   G = 16: l = l1 + 2 l2: exchange [n1][l] (pitch 18), radix 8 over l2,
-//           twiddle W_16^(l1 m1), exchange [n1][l1][m1] (pitches 18, 9),
-//           radix 2 over l1.
+//           twiddle W_16^(l1 m1), radix 2 over the lane pair l1 by shuffles.
 // The pitches put the 16 lanes of every half-warp on distinct banks for the
 // 8-byte accesses of each exchange (rows of a 128^3 warp are 72 apart, 8
 // modulo 16, and of a 64^3 warp 68, 4 modulo 16, so the rows sharing a
@@ -388,10 +397,6 @@ struct Cfg {
     static constexpr int RL = (N / 2 + 4) * 3;     // padded interleaved row (complex)
     static constexpr int XB = G == 4 ? 68 : (G == 8 ? 72 : 144);  // exchange block per row
     static constexpr int P1 = G == 16 ? 18 : 9;                   // [n1][l] pitch
-    // twiddle table [n1][l] pitch: the forward transform of G = 16 reads it
-    // with lane 2 n1 + l1 at column l1 + 2 l2, which a pitch of 16 would put
-    // on one bank for all eight n1
-    static constexpr int TP = G == 16 ? 18 : G;
 };
 
 template <int N>
@@ -404,11 +409,11 @@ struct Smem {
 // inverse (sign +): Z[l + G q] in v[q] -> grid order (layout above)
 template <int N>
 __device__ __forceinline__ void inv_g(cpx<float> (&v)[8], cpx<float>* xb,
-                                      const cpx<float>* __restrict__ t1, int l) {
+                                      const cpx<float> (&t1r)[8], int l) {
     constexpr int G = Cfg<N>::G, P1 = Cfg<N>::P1;
     dft<float, true, 8>(v);  // over q -> n1
 #pragma unroll
-    for (int n1 = 1; n1 < 8; ++n1) v[n1] = cmulc(v[n1], t1[n1 * Cfg<N>::TP + l]);  // W_M^{-n1 l}
+    for (int n1 = 1; n1 < 8; ++n1) v[n1] = cmulc(v[n1], t1r[n1]);  // W_M^{-n1 l}
     __syncwarp();
 #pragma unroll
     for (int n1 = 0; n1 < 8; ++n1) xb[n1 * P1 + l] = v[n1];
@@ -440,17 +445,17 @@ __device__ __forceinline__ void inv_g(cpx<float> (&v)[8], cpx<float>* xb,
 #pragma unroll
             for (int m1 = 1; m1 < 8; ++m1) v[m1] = mul_wr<float, true, 16>(v[m1], m1);  // W_16^{-m1}
         }
-        __syncwarp();
-#pragma unroll
-        for (int m1 = 0; m1 < 8; ++m1) xb[n1 * P1 + 9 * l1 + m1] = v[m1];
-        __syncwarp();
-        const int j = l & 1;
+        // lane j of the pair takes m1 = j + 2 i of both l1
+        cpx<float> own[4], got[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const cpx<float> a = xb[n1 * P1 + j + 2 * i];
-            const cpx<float> b = xb[n1 * P1 + 9 + j + 2 * i];
-            v[i] = a + b;  // m2 = 0
-            v[i + 4] = a - b;  // m2 = 1
+            own[i] = xw::pick(l1 != 0, v[2 * i + 1], v[2 * i]);
+            got[i] = xw::shfl_c(xw::pick(l1 != 0, v[2 * i], v[2 * i + 1]), 1);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[i] = own[i] + got[i];  // m2 = 0
+            v[i + 4] = l1 ? got[i] - own[i] : own[i] - got[i];  // m2 = 1
         }
     }
 }
@@ -458,7 +463,7 @@ __device__ __forceinline__ void inv_g(cpx<float> (&v)[8], cpx<float>* xb,
 // forward (sign -): grid order in -> Z[l + G q] in v[q]
 template <int N>
 __device__ __forceinline__ void fwd_g(cpx<float> (&v)[8], cpx<float>* xb,
-                                      const cpx<float>* __restrict__ t1, int l) {
+                                      const cpx<float> (&t1r)[8], int l) {
     constexpr int G = Cfg<N>::G, P1 = Cfg<N>::P1;
     if constexpr (G == 4) {
         cpx<float> a[4], b[4];
@@ -469,11 +474,6 @@ __device__ __forceinline__ void fwd_g(cpx<float> (&v)[8], cpx<float>* xb,
         }
         dft<float, false, 4>(a);  // over n2 -> k
         dft<float, false, 4>(b);
-#pragma unroll
-        for (int k = 1; k < 4; ++k) {
-            a[k] = cmul(a[k], t1[l * Cfg<N>::TP + k]);        // W_M^{n1 k}
-            b[k] = cmul(b[k], t1[(l + 4) * Cfg<N>::TP + k]);
-        }
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -482,34 +482,35 @@ __device__ __forceinline__ void fwd_g(cpx<float> (&v)[8], cpx<float>* xb,
         }
     } else if constexpr (G == 8) {
         dft<float, false, 8>(v);  // over n2 -> k (lane = n1)
-#pragma unroll
-        for (int k = 1; k < 8; ++k) v[k] = cmul(v[k], t1[k * Cfg<N>::TP + l]);  // W_M^{n1 k}, n1 = l
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < 8; ++k) xb[l * P1 + k] = v[k];
     } else {
-        const int n1 = l >> 1, j = l & 1;
-        __syncwarp();
+        const int n1 = l >> 1, l1 = l & 1;
+        // m1 = l1 + 2 i here; each lane of the pair takes its l1 of every m1
+        cpx<float> own[4], got[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const cpx<float> a = v[i], b = v[i + 4];
-            xb[n1 * P1 + j + 2 * i] = a + b;                                           // l1 = 0
-            xb[n1 * P1 + 9 + j + 2 * i] = mul_wr<float, false, 16>(a - b, j + 2 * i);  // l1 = 1
+            const cpx<float> sum = v[i] + v[i + 4], dif = v[i] - v[i + 4];
+            const cpx<float> rot = xw::pick(l1 != 0, mul_wr<float, false, 16>(dif, 1 + 2 * i),
+                                            mul_wr<float, false, 16>(dif, 2 * i));
+            own[i] = xw::pick(l1 != 0, rot, sum);
+            got[i] = xw::shfl_c(xw::pick(l1 != 0, sum, rot), 1);
         }
-        __syncwarp();
-        const int l1 = l & 1;
 #pragma unroll
-        for (int m1 = 0; m1 < 8; ++m1) v[m1] = xb[n1 * P1 + 9 * l1 + m1];
+        for (int i = 0; i < 4; ++i) {
+            v[2 * i] = xw::pick(l1 != 0, got[i], own[i]);
+            v[2 * i + 1] = xw::pick(l1 != 0, own[i], got[i]);
+        }
         dft<float, false, 8>(v);  // over m1 -> l2
-#pragma unroll
-        for (int l2 = 0; l2 < 8; ++l2) v[l2] = cmul(v[l2], t1[n1 * Cfg<N>::TP + l1 + 2 * l2]);  // W_M^{n1 k}
         __syncwarp();
 #pragma unroll
         for (int l2 = 0; l2 < 8; ++l2) xb[n1 * P1 + l1 + 2 * l2] = v[l2];
     }
     __syncwarp();
+    v[0] = xb[l];  // lane l takes spectrum column l
 #pragma unroll
-    for (int n1 = 0; n1 < 8; ++n1) v[n1] = xb[n1 * P1 + l];  // lane l takes spectrum column l
+    for (int n1 = 1; n1 < 8; ++n1) v[n1] = cmul(xb[n1 * P1 + l], t1r[n1]);  // W_M^{n1 l}
     dft<float, false, 8>(v);  // over n1 -> q
 }
 
@@ -526,7 +527,7 @@ __device__ __forceinline__ int grid_pair(int l, int i) {
 template <int N>
 __host__ __device__ constexpr size_t xwg_smem_bytes() {
     return (size_t)xwg::NWARP * sizeof(xwg::Smem<N>) +
-           (size_t)(N + 8 * xwg::Cfg<N>::TP) * sizeof(cpx<float>) + xwg::NWARP * 16;
+           (size_t)N * sizeof(cpx<float>) + xwg::NWARP * 16;
 }
 
 template <int N, bool WRITE_RU>
@@ -547,15 +548,13 @@ row_nonlin_wg(const Member<float>* __restrict__ mem, const Roles rl,
     extern __shared__ __align__(128) unsigned char xwg_smem_raw[];
     Smem<N>* ws = reinterpret_cast<Smem<N>*>(xwg_smem_raw);
     C* tw = reinterpret_cast<C*>(ws + NWARP);  // exp(-2 pi i m / N), m < N
-    C* t1 = tw + N;                            // [n1][l] = W_M^{n1 l}, pitch TP
-    unsigned long long* bars = reinterpret_cast<unsigned long long*>(t1 + 8 * CF::TP);
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(tw + N);
 
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     for (int i = tid; i < N; i += blockDim.x) tw[i] = tw_g[i];
-    for (int i = tid; i < 8 * G; i += blockDim.x) {
-        const int n1 = i / G, l = i % G;
-        t1[n1 * CF::TP + l] = tw_g[(2 * n1 * l) % N];
-    }
+    C t1r[8];  // W_M^{n1 l} of this lane
+#pragma unroll
+    for (int n1 = 0; n1 < 8; ++n1) t1r[n1] = tw_g[(2 * n1 * (lane % G)) % N];
     if (tid < 2 * NWARP) mbar_init(&bars[tid], 1);
     fence_mbar_init();
     __syncthreads();
@@ -679,7 +678,7 @@ row_nonlin_wg(const Member<float>* __restrict__ mem, const Roles rl,
                     v[q] = c2r_lo(a, st[3 * (M - k) + c], tw[k]);
                 }
             }
-            inv_g<N>(v, xb, t1, l);
+            inv_g<N>(v, xb, t1r, l);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 if (f < 3) U[c][i] = v[i];
@@ -708,20 +707,17 @@ row_nonlin_wg(const Member<float>* __restrict__ mem, const Roles rl,
             C v[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = U[c][i];
-            fwd_g<N>(v, xb, t1, l);
-            __syncwarp();
-#pragma unroll
-            for (int q = 0; q < 8; ++q) xb[l + G * q] = v[q];  // natural order
-            __syncwarp();
+            fwd_g<N>(v, xb, t1r, l);
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const int k = l + G * q;
+                const C zm = xw::mirror<G>(v, q, l);
                 if (k == 0) {
                     const C z0 = v[0];
                     so[c] = mk<float>(z0.x + z0.y, 0.f);
                     so[3 * M + c] = mk<float>(z0.x - z0.y, 0.f);
                 } else {
-                    so[3 * k + c] = r2c_lo(v[q], xb[M - k], tw[k]);
+                    so[3 * k + c] = r2c_lo(v[q], zm, tw[k]);
                 }
             }
         }

@@ -40,11 +40,6 @@ __host__ __device__ constexpr int xblock() {
     if constexpr (N == 512) return xw::XBUF;
     else return xwg::Cfg<N>::XB;
 }
-template <int N>
-__host__ __device__ constexpr int t1_pitch() {
-    if constexpr (N == 512) return xw::T1P;
-    else return xwg::Cfg<N>::TP;
-}
 // floats of a block of Q padded real rows, with room for the 8-byte shift
 template <int N>
 __host__ __device__ constexpr int real_floats() { return (rows<N>() * (N + 2) * 3 + 7) / 4 * 4; }
@@ -58,7 +53,7 @@ struct Smem {
 };
 template <int N>
 __host__ __device__ constexpr int table_len() {
-    return N + 8 * t1_pitch<N>() + (N == 512 ? 4 * xw::T2P : 0);
+    return N + (N == 512 ? 4 * xw::T2P : 0);
 }
 template <int N>
 __host__ __device__ constexpr size_t smem_bytes() {
@@ -66,16 +61,16 @@ __host__ __device__ constexpr size_t smem_bytes() {
 }
 
 template <int N>
-__device__ __forceinline__ void inverse(cpx<float> (&v)[8], cpx<float>* xb, const cpx<float>* t1,
+__device__ __forceinline__ void inverse(cpx<float> (&v)[8], cpx<float>* xb, const cpx<float> (&t1r)[8],
                                         const cpx<float>* t2, int l) {
-    if constexpr (N == 512) xw::inv256(v, xb, t1, t2, l);
-    else xwg::inv_g<N>(v, xb, t1, l);
+    if constexpr (N == 512) xw::inv256(v, xb, t1r, t2, l);
+    else xwg::inv_g<N>(v, xb, t1r, l);
 }
 template <int N>
-__device__ __forceinline__ void forward(cpx<float> (&v)[8], cpx<float>* xb, const cpx<float>* t1,
+__device__ __forceinline__ void forward(cpx<float> (&v)[8], cpx<float>* xb, const cpx<float> (&t1r)[8],
                                         const cpx<float>* t2, int l) {
-    if constexpr (N == 512) xw::fwd256(v, xb, t1, t2, l);
-    else xwg::fwd_g<N>(v, xb, t1, l);
+    if constexpr (N == 512) xw::fwd256(v, xb, t1r, t2, l);
+    else xwg::fwd_g<N>(v, xb, t1r, l);
 }
 // grid pair of register i of lane l
 template <int N>
@@ -90,7 +85,8 @@ struct Warp {
     int lane, grp, row, l;  // lane group, its row of the block, lane within it
     int odd;                // this lane takes odd x first (see the kernels)
     cpx<float>* xb;
-    const cpx<float>*tw, *t1, *t2;
+    const cpx<float>*tw, *t2;
+    cpx<float> t1r[8];      // W_M^{n1 l}
     unsigned long long* bar;
     int first, step, nblk;  // blocks of this warp
 };
@@ -103,15 +99,10 @@ __device__ __forceinline__ Warp<N> setup(unsigned char* smem, const cpx<float>* 
     constexpr int G = lanes<N>();
     Smem<N>* ws = reinterpret_cast<Smem<N>*>(smem);
     C* tw = reinterpret_cast<C*>(ws + NWARP);
-    C* t1 = tw + N;
-    C* t2 = t1 + 8 * t1_pitch<N>();
+    C* t2 = tw + N;
     unsigned long long* bars = reinterpret_cast<unsigned long long*>(tw + table_len<N>());
     const int tid = threadIdx.x, wid = tid >> 5;
     for (int i = tid; i < N; i += blockDim.x) tw[i] = tw_g[i];
-    for (int i = tid; i < 8 * G; i += blockDim.x) {
-        const int n1 = i / G, l = i % G;
-        t1[n1 * t1_pitch<N>() + l] = tw_g[(2 * n1 * l) % N];
-    }
     if constexpr (N == 512)
         if (tid < 32) t2[(tid >> 3) * xw::T2P + (tid & 7)] = tw_g[16 * ((tid >> 3) * (tid & 7))];
     if (tid < NWARP) mbar_init(&bars[tid], 1);
@@ -127,7 +118,8 @@ __device__ __forceinline__ Warp<N> setup(unsigned char* smem, const cpx<float>* 
     w.odd = N == 512 ? (w.l >> 1) & 1 : w.row & 1;
     w.xb = ws[wid].x + w.grp * xblock<N>();
     w.tw = tw;
-    w.t1 = t1;
+#pragma unroll
+    for (int n1 = 0; n1 < 8; ++n1) w.t1r[n1] = tw_g[(2 * n1 * w.l) % N];
     w.t2 = t2;
     w.bar = &bars[wid];
     w.nblk = nrows / rows<N>();
@@ -215,7 +207,7 @@ row_c2r_bulk(const Member<float>* __restrict__ mem, const Roles rl, float* __res
                     V[c][q] = c2r_lo(a, st[3 * (M - k) + c], w.tw[k]);
                 }
             }
-            inverse<N>(V[c], w.xb, w.t1, w.t2, w.l);
+            inverse<N>(V[c], w.xb, w.t1r, w.t2, w.l);
         }
         // the input rows are read and the previous output has left: next block
         if (blk + w.step < w.nblk) issue(blk + w.step);
@@ -322,23 +314,19 @@ row_r2c_bulk(const Member<float>* __restrict__ mem, const Roles rl, const float*
         C* so = S.cr + w.row * RL;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            forward<N>(V[c], w.xb, w.t1, w.t2, w.l);
-            __syncwarp();
-#pragma unroll
-            for (int q = 0; q < 8; ++q) w.xb[w.l + G * q] = V[c][q];  // natural order
-            __syncwarp();
+            forward<N>(V[c], w.xb, w.t1r, w.t2, w.l);
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const int k = w.l + G * q;
+                const C zm = xw::mirror<G>(V[c], q, w.l);
                 if (k == 0) {
                     const C z0 = V[c][0];
                     so[c] = mk<float>(z0.x + z0.y, 0.f);
                     so[3 * M + c] = mk<float>(z0.x - z0.y, 0.f);
                 } else {
-                    so[3 * k + c] = r2c_lo(V[c][q], w.xb[M - k], w.tw[k]);
+                    so[3 * k + c] = r2c_lo(V[c][q], zm, w.tw[k]);
                 }
             }
-            __syncwarp();
         }
         // padding points of the output row carry zeros
         for (int e = w.l; e < RL - 3 * (M + 1); e += G) so[3 * (M + 1) + e] = zero_c<float>();
