@@ -187,6 +187,31 @@ struct Prof {
     }
 };
 
+// Launch of a pass that may be scheduled while the launch before it on the
+// stream drains (programmatic dependent launch; every such kernel calls
+// pdl_wait() before it touches anything an earlier launch may write, fft.cuh).
+// `early` for short launches only, whose start-up shows: a step at 32^3 FP64 takes
+// 98 us instead of 138, at 64^3 FP32 170 instead of 206, at 128^3 FP64 755 instead
+// of 796; at 256^3 FP32, where the x pass's one block per SM comes up unevenly, it
+// lost (2461 against 2373 us), and so did a mixed ensemble with it everywhere.
+template <typename... KA, typename... A>
+static void launch(bool early, void (*kern)(KA...), dim3 grid, int block, size_t smem, cudaStream_t st,
+                   A... args) {
+    cudaLaunchAttribute at;
+    memset(&at, 0, sizeof(at));
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);  // an error stays for after_launch
+}
+
 static bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
 // A kernel whose bounded wait on its own bulk copies ran out sets
@@ -354,6 +379,10 @@ struct Engine {
     using C = cpx<T>;
     using Mem = Member<T>;
 
+    // launches of up to 2^22 grid points (a 128^3 grid, sixteen 64^3 members)
+    // may start while the launch before drains: launch()
+    static bool early(int nmem) { return (size_t)N * N * N * nmem <= ((size_t)1 << 22); }
+
     // one persistent launch of a column pass over nmem members, in the
     // schedule the autotuner chose for this grid, precision, pass and
     // member count
@@ -382,8 +411,8 @@ struct Engine {
         Prof pr(c, col_kind(MODE));
         // dynamic tile order where a launch has at least 8 tiles per CTA
         int* tctr = ntiles >= 8 * grid ? c->tctr : nullptr;
-        kern<<<grid, col_threads<T, N, MODE, S>(), smem, c->stream>>>(mem, rl, (const C*)c->tw, ntx,
-                                                                     kdom, tiles_per, ntiles, tctr);
+        launch(early(nmem), kern, grid, col_threads<T, N, MODE, S>(), smem, c->stream, mem, rl, (const C*)c->tw, ntx,
+               kdom, tiles_per, ntiles, tctr);
         return after_launch(c, "col_pass");
     }
 
@@ -450,9 +479,8 @@ struct Engine {
             const int nrows = rows_per * nmem;
             const int grid = std::min(c->nsm, (nrows + xw::NWARP - 1) / xw::NWARP);
             Prof pr(c, K_X);
-            kern<<<grid, xw::NWARP * 32, smem, c->stream>>>(
-                reinterpret_cast<const Member<float>*>(mem), rl,
-                reinterpret_cast<const cpx<float>*>(c->tw), rows_per, nrows);
+            launch(early(nmem), kern, grid, xw::NWARP * 32, smem, c->stream, reinterpret_cast<const Member<float>*>(mem),
+                   rl, reinterpret_cast<const cpx<float>*>(c->tw), rows_per, nrows);
             return after_launch(c, "row_nonlin_warp");
         } else if constexpr (MODE == RM_NONLIN && sizeof(T) == 4 && (N == 64 || N == 128 || N == 256)) {
             // FP32 64^3 - 256^3: warp-group x pass (xpass.cuh)
@@ -467,9 +495,8 @@ struct Engine {
             const int nblk = nrows / Q;
             const int grid = std::min(c->nsm, (nblk + xwg::NWARP - 1) / xwg::NWARP);
             Prof pr(c, K_X);
-            kern<<<grid, xwg::NWARP * 32, smem, c->stream>>>(
-                reinterpret_cast<const Member<float>*>(mem), rl,
-                reinterpret_cast<const cpx<float>*>(c->tw), rows_per, nrows);
+            launch(early(nmem), kern, grid, xwg::NWARP * 32, smem, c->stream, reinterpret_cast<const Member<float>*>(mem),
+                   rl, reinterpret_cast<const cpx<float>*>(c->tw), rows_per, nrows);
             return after_launch(c, "row_nonlin_wg");
         } else if constexpr (MODE == RM_NONLIN && rnl_fused<T, N>()) {
             constexpr size_t smem = rnl_smem_bytes<T, N>();
@@ -482,8 +509,8 @@ struct Engine {
             const int ntiles = tiles_per * nmem;
             const int grid = std::min(ntiles, c->nsm * rnl_ctas<T, N>());
             Prof pr(c, K_X);
-            kern<<<grid, rnl_threads<T, N>(), smem, c->stream>>>(mem, rl, (const C*)c->tw, tiles_per,
-                                                         ntiles);
+            launch(early(nmem), kern, grid, rnl_threads<T, N>(), smem, c->stream, mem, rl, (const C*)c->tw, tiles_per,
+                   ntiles);
             return after_launch(c, "row_nonlin");
         }
         if constexpr ((MODE == RM_C2R || MODE == RM_R2C) && sizeof(T) == 4 && xr::supported<N>()) {
@@ -507,7 +534,7 @@ struct Engine {
         const int ntiles = tiles_per * nmem;
         const int grid = std::min(ntiles, c->nsm * ROW_CTAS);
         Prof pr(c, K_X);
-        kern<<<grid, ROW_THREADS, smem, c->stream>>>(mem, rl, (const C*)c->tw, tiles_per, ntiles);
+        launch(early(nmem), kern, grid, ROW_THREADS, smem, c->stream, mem, rl, (const C*)c->tw, tiles_per, ntiles);
         return after_launch(c, "row_pass");
     }
 
@@ -523,15 +550,14 @@ struct Engine {
         const int nblk = nrows / xr::rows<N>();
         const int grid = std::min(c->nsm, (nblk + xr::NWARP - 1) / xr::NWARP);
         Prof pr(c, K_X);
-        kern<<<grid, xr::NWARP * 32, smem, c->stream>>>(mem, rl, user,
-                                                        reinterpret_cast<const cpx<float>*>(c->tw),
-                                                        N * N, nrows);
+        launch(early(nmem), kern, grid, xr::NWARP * 32, smem, c->stream, mem, rl, user,
+               reinterpret_cast<const cpx<float>*>(c->tw), N * N, nrows);
         return after_launch(c, "row_bulk");
     }
 
     static int symmetrize(bfg_ctx* c, const Mem* mem, int nmem, int bufi) {
         Prof pr(c, K_KSPACE);
-        symmetrize_kernel<T, N><<<dim3((N * N + 255) / 256, nmem), 256, 0, c->stream>>>(mem, bufi);
+        launch(early(nmem), symmetrize_kernel<T, N>, dim3((N * N + 255) / 256, nmem), 256, 0, c->stream, mem, bufi);
         return after_launch(c, "symmetrize");
     }
 

@@ -90,6 +90,17 @@ __host__ __device__ __forceinline__ cpx<T> rot90(cpx<T> a) {
     return INV ? mk<T>(-a.y, a.x) : mk<T>(a.y, -a.x);
 }
 
+// --------------------------------------- programmatic dependent launch --
+// The passes are launched so that the next one may be scheduled while this one
+// drains (launch() in bfps_b200.cu): its blocks come up as this one's leave,
+// load their tables, and wait in pdl_wait() until every earlier launch of the
+// stream has completed and its writes are visible.  Nothing but tables that are
+// written once per context is read before that, and nothing is written.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ------------------------------------------------------ async copies --
 // cp.async (global -> shared, bypassing registers), PTX ISA 7.0+.
 __device__ __forceinline__ unsigned smem_u32(const void* p) {

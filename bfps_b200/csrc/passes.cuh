@@ -648,6 +648,8 @@ col_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
     constexpr size_t nxp3 = (size_t)(N / 2 + 4) * 3;
     const int tid = threadIdx.x;
     for (int i = tid; i < N; i += NT) tw[i] = tw_g[i];
+    pdl_wait();
+    pdl_release();
 
     // tile t: member t / tiles_per, then (a, kx-tile) with the kx-tile fastest
     // (ntx kx-tiles; rows a with |a| <= kdom where kdom >= 0, else all).
@@ -1050,6 +1052,8 @@ row_pass(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __rest
         // padding columns of the output rows are written out: start them at 0
         for (int i = tid; i < ROWS * RL; i += ROW_THREADS) outr[i] = zero_c<T>();
     }
+    pdl_wait();
+    pdl_release();
 
     // tile t: member t / tiles_per, then ROWS consecutive rows
     int t = blockIdx.x;
@@ -1349,6 +1353,8 @@ row_nonlin(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __re
     }
     if constexpr (WRITE_RU)
         for (int i = tid; i < M; i += RNL_THREADS) posn[i] = dif_position<M, MRR>(i);
+    pdl_wait();
+    pdl_release();
 
     // kx columns that the rows of a member hold on each side (read again only
     // where the member changes)
@@ -1665,6 +1671,8 @@ template <typename T, int N>
 __global__ void symmetrize_kernel(const Member<T>* __restrict__ mem, int bufi) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= N * N) return;
+    pdl_wait();
+    pdl_release();
     cpx<T>* s = mem[blockIdx.y].buf[bufi];
     const int nxp = N / 2 + 4;
     const int ky = e / N, kz = e % N;

@@ -189,6 +189,8 @@ row_nonlin_warp(const Member<float>* __restrict__ mem, const Roles rl,
     if (tid < 2 * NWARP) mbar_init(&bars[tid], 1);
     fence_mbar_init();
     __syncthreads();
+    pdl_wait();
+    pdl_release();
 
     Smem<N>& S = ws[wid];
     // bars[2 w]: the u row in su, bars[2 w + 1]: the w row in sw
@@ -558,6 +560,8 @@ row_nonlin_wg(const Member<float>* __restrict__ mem, const Roles rl,
     if (tid < 2 * NWARP) mbar_init(&bars[tid], 1);
     fence_mbar_init();
     __syncthreads();
+    pdl_wait();
+    pdl_release();
 
     Smem<N>& S = ws[wid];
     unsigned long long* bar_u = &bars[2 * wid];

@@ -108,6 +108,8 @@ __device__ __forceinline__ Warp<N> setup(unsigned char* smem, const cpx<float>* 
     if (tid < NWARP) mbar_init(&bars[tid], 1);
     fence_mbar_init();
     __syncthreads();
+    pdl_wait();
+    pdl_release();
     Warp<N> w;
     w.lane = tid & 31;
     w.grp = w.lane / G;
