@@ -71,9 +71,13 @@ def algorithmic_bytes(cfg):
     U = N^2 (N+2) P is one scalar field (real padded or half-spectrum complex).
     Step model (2-pass fused): 105 U for the IF-RK3 step; tracers add
     n * 24 * (k+2) + 6 N^3 P (write real u once, read it once in the gather).
-    Per launch of this engine's kernels (what each must move at least):
-    IZ 9U, IY 12U, X 9U (+ 3 N^3 P when it also writes the real velocity),
-    FY 6U, FZ 9U (stage 1) / 12U (stages 2, 3), tracers n*24*(k+2) + 3 N^3 P.
+    Per launch of this engine's kernels (what each must move at least): from
+    128^3 up the passes leave out the modes outside kM, so a state-layout field
+    counts s U per component (the sphere |k| <= kM of the half spectrum), a field
+    between the z and y passes d U (its disc of (kx, ky) columns), around the x
+    pass x U (kx columns): IZ 3s + 6d, IY 6d + 6x, X 9x (+ 3 N^3 P when it also
+    writes the real velocity), FY 3x + 3d, FZ 3d + 6s (stage 1) / 9s (stages 2,
+    3: two RK operands), tracers n*24*(k+2) + 3 N^3 P.
     """
     n = cfg["n"]
     P = 4 if cfg["precision"] == "single" else 8
@@ -82,12 +86,16 @@ def algorithmic_bytes(cfg):
     nt = cfg["ntracers"]
     real3 = 3 * n ** 3 * P
     step = 105 * U + nt * 24 * (k + 2) + 2 * real3
+    x = d = s = 1.0
+    if n >= 128:
+        x = (n // 2 - 1 if cfg["dealias"] == 1 else n // 3 - 1) / (n / 2)
+        d, s = math.pi / 4 * x ** 2, math.pi / 6 * x ** 3
     per_launch = {
-        "IZ": 9 * U,
-        "IY": 12 * U,
-        "X": 9 * U + (real3 / 3.0 if nt else 0.0),
-        "FY": 6 * U,
-        "FZ": (9 * U + 12 * U + 12 * U) / 3.0,
+        "IZ": (3 * s + 6 * d) * U,
+        "IY": (6 * d + 6 * x) * U,
+        "X": 9 * x * U + (real3 / 3.0 if nt else 0.0),
+        "FY": (3 * x + 3 * d) * U,
+        "FZ": (3 * d + 8 * s) * U,
         "kspace": 0.0,
         "tracers": nt * 24 * (k + 2) + real3,
         "stats": 0.0,
@@ -97,9 +105,9 @@ def algorithmic_bytes(cfg):
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of one launch
 # divided by its algorithmic bytes, from the ncu captures summarised under
-# profiles/ (256^3 FP32 passes; tracer kernel at 4e6 tracers on 256^3).
+# profiles/ (256^3 FP32 stage 1 passes; tracer kernel at 4e6 tracers on 256^3).
 # Traffic at another size is taken to scale with the algorithmic bytes.
-TRAFFIC_RATIO = {"X": 0.951, "IZ": 0.931, "IY": 0.948, "FY": 0.886, "FZ": 0.744, "tracers": 0.983}
+TRAFFIC_RATIO = {"X": 0.954, "IZ": 0.953, "IY": 0.972, "FY": 0.896, "FZ": 1.03, "tracers": 0.983}
 
 
 class ClockSampler:
