@@ -123,7 +123,8 @@ __host__ __device__ inline int tracer_split(int64_t n, int nb) {
 // the others three rows, four blocks (1e5 tracers, n = 2, m = 2, 256^3: 75 us;
 // one row and six blocks 100, two rows and five 94; six rows 76).  FP64: two
 // rows, three blocks (50001 tracers, n = 4, m = 1, 256^3: 190 us; one row and
-// four blocks 251, three rows 263, four rows and two blocks 217).
+// four blocks 251, three rows 263, four rows and two blocks 217; as built it takes
+// 124 registers, so four blocks fit: at 129 it was 10 % slower).
 template <typename T, int NB>
 __host__ __device__ constexpr int tracer_row_unroll() {
     return sizeof(T) == 4 ? (NB == 3 ? 2 * NB + 2 : 3) : 2;
@@ -147,6 +148,65 @@ __device__ __forceinline__ double group_sum(double v, unsigned gmask) {
     return v;
 }
 
+#ifndef BFG_TRACER_ROWSUM_F64
+#define BFG_TRACER_ROWSUM_F64 0
+#endif
+template <typename T>
+using row_sum_t =
+    typename std::conditional<sizeof(T) == 8 || BFG_TRACER_ROWSUM_F64 != 0, double, float>::type;
+
+// The sum of row_gather from the stencil's points alone, with scalar loads: lane
+// j takes the points ix = j, j + L, ... of each row (stencils across the periodic
+// x boundary, and resum below).
+template <typename T, int NB, int L, int U>
+__device__ __forceinline__ void point_gather(const T* __restrict__ ru, int N, const int* g, int x0,
+                                             const double* wx, const double* wy, const double* wz,
+                                             int j, int z0, int zs, unsigned gmask, double& a0,
+                                             double& a1, double& a2) {
+    using SumT = row_sum_t<T>;
+    constexpr int NP = 2 * NB + 2;
+    constexpr int PPL = (NP + L - 1) / L;  // points per lane
+    const size_t rowN = (size_t)N;
+    SumT wj[PPL];
+    int xj[PPL];
+#pragma unroll
+    for (int m = 0; m < PPL; ++m) {
+        const int ix = j + L * m;
+        SumT w = 0;
+#pragma unroll
+        for (int pt = 0; pt < NP; ++pt) w = ix == pt ? (SumT)wx[pt] : w;
+        wj[m] = w;
+        xj[m] = ix < NP ? wrap_once(x0 + ix, N) : -1;
+    }
+    double A[3] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+    for (int iz = z0; iz < NP; iz += zs) {
+        const int z = wrap_once(g[2] - NB + iz, N);
+        const double bz = wz[iz];
+#pragma unroll(U)
+        for (int iy = 0; iy < NP; ++iy) {
+            const int y = wrap_once(g[1] - NB + iy, N);
+            const T* row = ru + ((size_t)z * rowN + y) * rowN * 3;
+            SumT s0 = 0, s1 = 0, s2 = 0;
+#pragma unroll
+            for (int m = 0; m < PPL; ++m) {
+                if (xj[m] >= 0) {
+                    s0 = fma((SumT)row[xj[m] * 3 + 0], wj[m], s0);
+                    s1 = fma((SumT)row[xj[m] * 3 + 1], wj[m], s1);
+                    s2 = fma((SumT)row[xj[m] * 3 + 2], wj[m], s2);
+                }
+            }
+            const double bzy = bz * wy[iy];
+            A[0] = fma(bzy, (double)s0, A[0]);
+            A[1] = fma(bzy, (double)s1, A[1]);
+            A[2] = fma(bzy, (double)s2, A[2]);
+        }
+    }
+    a0 = group_sum<L>(A[0], gmask);
+    a1 = group_sum<L>(A[1], gmask);
+    a2 = group_sum<L>(A[2], gmask);
+}
+
 // Lane j (0..L-1) of a lane group reads vectors j, j + L, ... of each row of
 // the group's z planes (iz = z0, z0 + zs, ...).  FP32 field (precision form):
 // the x sums of the stencil rows run in FP32 with the x weights rounded to
@@ -155,17 +215,14 @@ __device__ __forceinline__ double group_sum(double v, unsigned gmask) {
 // FP64 field: all of it in FP64.  Word i of the row segment read from the
 // aligned-down start belongs to point (i - off) / 3, component
 // (i - off) mod 3, so each lane's x weights are shifted once per tracer and its
-// sums are kept per word phase i mod 3, mapped to components at the end.
-#ifndef BFG_TRACER_ROWSUM_F64
-#define BFG_TRACER_ROWSUM_F64 0
-#endif
+// sums are kept per word phase i mod 3, mapped to components at the end.  Words
+// of a vector beside the stencil enter with weight zero (see tracer_one).
 template <typename T, int NB, int L>
 __device__ __forceinline__ void row_gather(const T* __restrict__ ru, int N, const int* g, int x0,
                                            const double* wx, const double* wy, const double* wz,
                                            int j, int z0, int zs, unsigned gmask, double& a0,
                                            double& a1, double& a2) {
-    using SumT =
-        typename std::conditional<sizeof(T) == 8 || BFG_TRACER_ROWSUM_F64 != 0, double, float>::type;
+    using SumT = row_sum_t<T>;
     constexpr int NP = 2 * NB + 2;
     constexpr int VW = 32 / (int)sizeof(T);              // values per vector
     constexpr int NVMAX = (3 * NP + 2 * (VW - 1)) / VW;  // vectors covering any alignment
@@ -232,48 +289,32 @@ __device__ __forceinline__ void row_gather(const T* __restrict__ ru, int N, cons
         a1 = k0 == 0 ? G[1] : (k0 == 1 ? G[2] : G[0]);
         a2 = k0 == 0 ? G[2] : (k0 == 1 ? G[0] : G[1]);
     } else {
-        // stencil across the periodic x boundary: lane j takes the points
-        // ix = j, j + L, ... with scalar loads
-        constexpr int PPL = (NP + L - 1) / L;  // points per lane
-        SumT wj[PPL];
-        int xj[PPL];
-#pragma unroll
-        for (int m = 0; m < PPL; ++m) {
-            const int ix = j + L * m;
-            SumT w = 0;
-#pragma unroll
-            for (int pt = 0; pt < NP; ++pt) w = ix == pt ? wxf[pt] : w;
-            wj[m] = w;
-            xj[m] = ix < NP ? wrap_once(x0 + ix, N) : -1;
-        }
-        double A[3] = {0.0, 0.0, 0.0};
-#pragma unroll 1
-        for (int iz = z0; iz < NP; iz += zs) {
-            const int z = wrap_once(g[2] - NB + iz, N);
-            const double bz = wz[iz];
-#pragma unroll(tracer_row_unroll<T, NB>())
-            for (int iy = 0; iy < NP; ++iy) {
-                const int y = wrap_once(g[1] - NB + iy, N);
-                const T* row = ru + ((size_t)z * rowN + y) * rowN * 3;
-                SumT s0 = 0, s1 = 0, s2 = 0;
-#pragma unroll
-                for (int m = 0; m < PPL; ++m) {
-                    if (xj[m] >= 0) {
-                        s0 = fma((SumT)row[xj[m] * 3 + 0], wj[m], s0);
-                        s1 = fma((SumT)row[xj[m] * 3 + 1], wj[m], s1);
-                        s2 = fma((SumT)row[xj[m] * 3 + 2], wj[m], s2);
-                    }
-                }
-                const double bzy = bz * wy[iy];
-                A[0] = fma(bzy, (double)s0, A[0]);
-                A[1] = fma(bzy, (double)s1, A[1]);
-                A[2] = fma(bzy, (double)s2, A[2]);
-            }
-        }
-        a0 = group_sum<L>(A[0], gmask);
-        a1 = group_sum<L>(A[1], gmask);
-        a2 = group_sum<L>(A[2], gmask);
+        point_gather<T, NB, L, tracer_row_unroll<T, NB>()>(ru, N, g, x0, wx, wy, wz, j, z0, zs, gmask,
+                                                           a0, a1, a2);
     }
+}
+
+// u at one tracer from the stencil's points alone; cell and weights are worked
+// out again (the position read anew), so that none of them has to stay in
+// registers during row_gather.
+template <typename T, int NB, int MM>
+__device__ __forceinline__ void resum(const PParams& pp, const T* __restrict__ ru,
+                                      const volatile double* pos, int sub, int z0, int zs,
+                                      unsigned gmask, double* acc) {
+    constexpr int NP = 2 * NB + 2;
+    constexpr int L = tracer_lanes<T>();
+    int g[3];
+    double fr[3], wx[NP], wy[NP], wz[NP];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) cell_of(pos[d], pp.box[d], pp.hstep[d], pp.N, &g[d], &fr[d]);
+    beta_weights<NB, MM>(fr[0], wx);
+    beta_weights<NB, MM>(fr[1], wy);
+    beta_weights<NB, MM>(fr[2], wz);
+    point_gather<T, NB, L, 1>(ru, pp.N, g, g[0] - NB, wx, wy, wz, sub % L, z0, zs, gmask, acc[0],
+                              acc[1], acc[2]);
+    for (int o = L; o < L * zs; o *= 2)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) acc[d] += __shfl_xor_sync(gmask, acc[d], o);
 }
 
 // tracer i of one system, lane `sub` of its pp.split groups of
@@ -299,6 +340,16 @@ __device__ __forceinline__ void tracer_one(const PParams& pp, const T* __restric
     beta_weights<NB, MM>(fr[1], wy);
     beta_weights<NB, MM>(fr[2], wz);
 
+    // lane sub < L finishes components sub, sub + L, ...; only their coordinates
+    // stay in registers during the gather
+    constexpr int CPL = (3 + L - 1) / L;
+    double xd[CPL];
+#pragma unroll
+    for (int m = 0; m < CPL; ++m) {
+        const int d = sub + L * m;
+        xd[m] = d == 0 ? p[0] : (d == 1 ? p[1] : p[2]);
+    }
+
     double acc[3] = {0.0, 0.0, 0.0};
     const int z0 = tracer_splits<T>(NB) ? sub / L : 0, zs = tracer_splits<T>(NB) ? pp.split : 1;
     row_gather<T, NB, L>(ru, N, g, g[0] - NB, wx, wy, wz, sub % L, z0, zs, gmask, acc[0], acc[1],
@@ -307,23 +358,28 @@ __device__ __forceinline__ void tracer_one(const PParams& pp, const T* __restric
     for (int o = L; o < L * zs; o *= 2)
 #pragma unroll
         for (int d = 0; d < 3; ++d) acc[d] += __shfl_xor_sync(gmask, acc[d], o);
-    const int j = sub;  // lane j < L finishes components j, j + L, ...
-    if (j >= L) return;
-    if (!pp.move) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-            if (d % L == j) sample_out[i * 3 + d] = acc[d];
-        return;
-    }
-    const int ns = pp.nsteps;
+    // Row vectors also hold words beside the stencil, which entered with weight
+    // zero: an infinity or NaN among them makes the sum NaN.  So a sum that is not
+    // finite is formed again from the stencil's points alone (the sums are the
+    // same on all lanes of the tracer, so they all come here together).
+    if (!(isfinite(acc[0]) && isfinite(acc[1]) && isfinite(acc[2])))
+        resum<T, NB, MM>(pp, ru, pos + i * 3, sub, z0, zs, gmask, acc);
+    if (sub >= L) return;
     const size_t slot = (size_t)pp.n * 3;
     const double dt = pp.dt;
+    const int ns = pp.nsteps;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        if (d % L != j) continue;
+    for (int m = 0; m < CPL; ++m) {
+        const int d = sub + L * m;
+        if (d >= 3) continue;
+        const double u = d == 0 ? acc[0] : (d == 1 ? acc[1] : acc[2]);
+        if (!pp.move) {
+            sample_out[i * 3 + d] = u;
+            continue;
+        }
         double* h0 = hist + (size_t)pp.head * slot + i * 3 + d;
         double r[6];
-        r[0] = acc[d];
+        r[0] = u;
         if (pp.accum) r[0] += *h0;
         *h0 = r[0];
 #pragma unroll
@@ -335,7 +391,7 @@ __device__ __forceinline__ void tracer_one(const PParams& pp, const T* __restric
                 r[k] = hist[(size_t)sl * slot + i * 3 + d];
             }
         }
-        double x = p[d];
+        double x = xd[m];
         switch (pp.order) {
             case 1: x += dt * r[0]; break;
             case 2: x += dt * (3. * r[0] - r[1]) / 2.; break;

@@ -1,7 +1,8 @@
 """Lanes and lane groups of the tracer gather: tracer counts on both sides of
 every change of the split (tracer_split: 4 lanes a row and up to 37888 threads in
 FP64, 2 lanes in FP32), all stencil widths, stencils across the periodic
-boundary at every lane, against the oracle; the same bits alone and batched."""
+boundary at every lane, values beside a stencil, against the oracle; the same
+bits alone and batched."""
 import numpy as np
 import pytest
 
@@ -51,6 +52,40 @@ def test_sample_at_split_edges(flow, precision, nm, count):
     tol = 1e-13 * 12 if precision == "double" else 2e-6
     assert np.abs(got - want).max() <= tol * np.abs(field).max()
     ps.close()
+    ve.close()
+
+
+@pytest.mark.parametrize("precision", ["double", "single"])
+@pytest.mark.parametrize("nm,count", [((1, 1), 9), ((2, 0), 2500), ((3, 2), 40), ((4, 1), 40), ((5, 1), 9)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_values_beside_the_stencil_do_not_enter(flow, precision, nm, count, bad):
+    """Not-finite planes of points right beside the stencil, at every alignment
+    of the stencil's row, leave the sample as it is; inside, they reach it."""
+    from bfps_b200.solver import vorticity_equation, particles_system
+    _, ur = flow
+    n = nm[0]
+    ve = vorticity_equation(N, precision=precision)
+    h = 2 * np.pi / N
+    rng = np.random.default_rng(count)
+    # cells 14..21 start their rows at every word of a vector (8 FP32, 4 FP64);
+    # cell 1: across the boundary (n > 1)
+    for cell in [1] + list(range(14, 22)):
+        pos = rng.random((count, 3)) * 2 * np.pi
+        pos[:, 0] = (cell + 0.1 + 0.8 * rng.random(count)) * h
+        pos[-1, 0] -= h  # the last tracer's stencil holds the left plane
+        field = np.zeros(ve.rshape, ve.rdtype)
+        field[:, :, :N] = ur
+        clean = field[:, :, :N].astype(np.float64)
+        field[:, :, [(cell - n - 1) % N, (cell + n + 2) % N]] = bad
+        ve.set_rvelocity(field)
+        ps = particles_system(ve, pos, nm[0], nm[1], nsteps=2)
+        got = ps.sample_velocity()
+        ps.close()
+        want = P.sample(clean, pos, nm[0], nm[1], P.Geometry(N, N, N))
+        # as in test_sample_at_split_edges
+        tol = 1e-13 * 12 if precision == "double" else 2e-6
+        assert np.abs(got - want)[:-1].max() <= tol * np.abs(clean).max(), cell
+        assert not np.isfinite(got[-1]).any()
     ve.close()
 
 
