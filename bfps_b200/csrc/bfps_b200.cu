@@ -995,7 +995,7 @@ static int ensure_ru(bfg_ctx* c) {
 template <typename T, int NB, int MM>
 static int launch_tracers(bfg_ctx* c, const PParams& pp, bfg_pctx* p, double* out,
                           cudaStream_t st, const void* field) {
-    const int tpb = tracers_per_block<T>(pp.split);
+    const int tpb = tracers_per_block<T>(pp.split, NB, pp.many);
     const unsigned blocks = (unsigned)((p->n + tpb - 1) / tpb);
     if (blocks == 0) return 0;
     Prof pr(c, K_TRACER, st);
@@ -1036,6 +1036,8 @@ static PParams pparams(const bfg_pctx* p, double dt, int move) {
     pp.move = move;
     pp.split = c->real_bytes == 4 ? tracer_split<float>(p->n, p->neighbours)
                                   : tracer_split<double>(p->n, p->neighbours);
+    pp.many = c->real_bytes == 4 ? tracer_many<float>(p->n, p->neighbours)
+                                 : tracer_many<double>(p->n, p->neighbours);
     pp.dt = dt;
     return pp;
 }
@@ -2362,8 +2364,9 @@ static int ens_prepare(bfg_ens* e) {
         ts.pos = p->pos;
         ts.hist = p->hist;
         sets.push_back(ts);
-        const int64_t tpb = e->real_bytes == 4 ? tracers_per_block<float>(ts.pp.split)
-                                               : tracers_per_block<double>(ts.pp.split);
+        const int64_t tpb = e->real_bytes == 4
+                                ? tracers_per_block<float>(ts.pp.split, p->neighbours, ts.pp.many)
+                                : tracers_per_block<double>(ts.pp.split, p->neighbours, ts.pp.many);
         start.push_back(start.back() + (p->n + tpb - 1) / tpb);
         e->batched.push_back(i);
     }

@@ -33,6 +33,7 @@ struct PParams {
     int accum;        // rhs[0] += u(x) instead of =
     int move;         // 0: sample only (into out), 1: full loop
     int split;        // lane groups of one tracer that share its z planes (tracer_split)
+    int many;         // the form for many tracers (tracer_many)
     double dt;
 };
 
@@ -80,28 +81,33 @@ __device__ __forceinline__ void ld_32b(const double* p, double* v) {  // four do
 
 constexpr int TRACER_THREADS = 128;
 
-// Lanes that share one stencil row: two for FP32 fields, four for FP64 fields.
-// A row is read as 32-byte sectors from its aligned-down start (up to four in
-// FP32, nine in FP64 for n = 4).  With one lane per tracer the gather is bound
-// by L1 wavefronts (about one per sector, as each lane's sector lies in another
-// line); with the sectors of a row spread over the lanes of one load, a
+// Lanes that share one stencil row: two for FP32 fields, four for FP64 fields
+// (n = 1: two).  A row is read as 32-byte sectors from its aligned-down start (up
+// to four in FP32, nine in FP64 for n = 4).  With one lane per tracer the gather is
+// bound by L1 wavefronts (about one per sector, as each lane's sector lies in
+// another line); with the sectors of a row spread over the lanes of one load, a
 // wavefront serves them all, and only the per-row address and FP64 work grows.
 // Measured on B200, FP32 (4e6 tracers, n = 3, m = 2, 512^3): 3.26 ms with one
 // lane, 2.70 ms with two, 4.47 ms with four (issue bound).  FP64 (50001
 // tracers, n = 4, m = 1, 256^3): 490 us with one lane, 250 us with four (190 us
-// with the loop shape below).
+// with the loop shape below).  Narrow FP64 stencils have few sectors a row, so the
+// lanes' own work weighs more: n = 1, 1e6 tracers, 128^3: 347 us with four lanes,
+// 260 with two; n = 2: 5000 tracers 15 us with four lanes, 21 with two, but 1e6
+// in cell order 707 against 610.  So n = 2 takes two for many tracers.
 template <typename T>
-__host__ __device__ constexpr int tracer_lanes() {
-    return sizeof(T) == 4 ? 2 : 4;
+__host__ __device__ constexpr int tracer_lanes(int nb, bool many) {
+    return sizeof(T) == 4 || nb == 1 || (nb == 2 && many) ? 2 : 4;
 }
 // Few tracers leave the chip waiting for one dependent row after another: then
 // up to eight lane groups share a tracer, group g taking the z planes g, g +
-// split, ..., as long as all groups together are no more than 256 threads per
-// SM (the gather of more threads is bound by throughput, and every group
-// repeats the cell and weight arithmetic).  It depends on the number of tracers
-// only, so a system sums in the same order alone and in an ensemble.  The FP32
-// n = 3 gather, unrolled up to its register limit, is not split (the runtime
-// plane stride spilled there: 2.47 -> 2.55 ms for 4e6 tracers).
+// split, ..., as long as all groups together are no more than 256 threads on each
+// of 148 SMs (the gather of more threads is bound by throughput, and every group
+// repeats the cell and weight arithmetic).  Lanes and split depend on the number
+// of tracers only, not on the device, so a system sums in the same order alone
+// and in an ensemble, everywhere.  The FP32 n = 3 gather is not split at any
+// count: the runtime plane stride spilled in its kernel, unrolled up to the
+// register limit (4e6 tracers 2.47 -> 2.55 ms), and a second form of it for few
+// tracers has not been tried.
 // 1024 tracers, FP64, n = 2: 45 us with one lane per tracer, 14 us with
 // four lanes a row and up to eight groups.
 template <typename T>
@@ -110,32 +116,51 @@ __host__ __device__ constexpr bool tracer_splits(int nb) {
 }
 template <typename T>
 __host__ __device__ inline int tracer_split(int64_t n, int nb) {
-    const int lanes = tracer_lanes<T>(), planes = 2 * nb + 2;
+    const int lanes = tracer_lanes<T>(nb, false), planes = 2 * nb + 2;
     int r = 1;
     if (!tracer_splits<T>(nb)) return r;
     while (r < 8 && 2 * r <= planes && 2 * r * lanes <= 32 && n * lanes * 2 * r <= 148 * 256) r *= 2;
     return r;
 }
+// Many tracers (PParams::many; never split): the two narrow gathers that lose by
+// the runtime plane stride, or want fewer lanes, have a form of their own for them
+// in the same kernel.  128^3, us for 1e5 / 2e5 / 1e6 tracers, common form against
+// own form: FP32 n = 1 32 / 54 / 236 against 29 / 48 / 205; FP64 n = 2 79 / 147 / 701
+// against 80 / 147 / 641.
+constexpr int64_t TRACERS_MANY = 1 << 17;
+template <typename T>
+__host__ __device__ constexpr bool tracer_many_form(int nb) {
+    return sizeof(T) == 4 ? nb == 1 : nb == 2;
+}
+template <typename T>
+__host__ __device__ inline int tracer_many(int64_t n, int nb) {
+    return tracer_many_form<T>(nb) && n > TRACERS_MANY ? 1 : 0;
+}
 // The gather waits for its rows (long scoreboard): rows of the y loop are
 // unrolled so that several are in flight, and the kernels are given the
-// registers for that.  FP32: n = 3 its eight rows, four blocks per SM (4e6
-// tracers, 512^3: 2.43 ms; five blocks 2.47-2.52, four rows and six blocks 2.57);
-// the others three rows, four blocks (1e5 tracers, n = 2, m = 2, 256^3: 75 us;
-// one row and six blocks 100, two rows and five 94; six rows 76).  FP64: two
-// rows, three blocks (50001 tracers, n = 4, m = 1, 256^3: 190 us; one row and
-// four blocks 251, three rows 263, four rows and two blocks 217; as built it takes
-// 124 registers, so four blocks fit: at 129 it was 10 % slower).
+// registers for that (us or ms by rows and blocks per SM):
+//   FP32, n = 3: eight rows, four blocks (4e6 tracers, 512^3: 2.43 ms; five blocks
+//   2.47-2.52, four rows and six blocks 2.57); n = 2: three, four (1e5 tracers,
+//   256^3: 75 us; one and six 100, two and five 94, six rows 76); n = 1: two, six
+//   (1e6, 128^3: 205 us; three and four 234, two and eight 197 but 5000 tracers 12
+//   against 11); n = 4: two, four (1e6, 128^3: 1.68 ms; three and four 1.77, one and
+//   four 1.93); n = 5: three, four.
+//   FP64: two rows, and three for n = 2 (1e6, 128^3: 641 us; two 659); four blocks,
+//   n = 1 five (1e6, 128^3: 260 us; four 286).  n = 4, 50001 tracers, 256^3: 190 us;
+//   one row 251, three rows and three blocks 263, four rows and two blocks 217.
 template <typename T, int NB>
 __host__ __device__ constexpr int tracer_row_unroll() {
-    return sizeof(T) == 4 ? (NB == 3 ? 2 * NB + 2 : 3) : 2;
+    if (sizeof(T) == 8) return NB == 2 ? 3 : 2;
+    return NB == 3 ? 2 * NB + 2 : (NB == 1 || NB == 4 ? 2 : 3);
 }
 template <typename T, int NB>
 __host__ __device__ constexpr int tracer_min_blocks() {
-    return sizeof(T) == 8 ? 3 : 4;
+    if (NB == 1) return sizeof(T) == 4 ? 6 : 5;
+    return 4;
 }
 template <typename T>
-__host__ __device__ inline int tracers_per_block(int split) {
-    return TRACER_THREADS / (tracer_lanes<T>() * split);
+__host__ __device__ inline int tracers_per_block(int split, int nb, bool many) {
+    return TRACER_THREADS / (tracer_lanes<T>(nb, many) * split);
 }
 
 // sum of v over the L lanes of a tracer group, pairwise ((l0 + l1) + (l2 +
@@ -297,12 +322,11 @@ __device__ __forceinline__ void row_gather(const T* __restrict__ ru, int N, cons
 // u at one tracer from the stencil's points alone; cell and weights are worked
 // out again (the position read anew), so that none of them has to stay in
 // registers during row_gather.
-template <typename T, int NB, int MM>
+template <typename T, int NB, int MM, int L>
 __device__ __forceinline__ void resum(const PParams& pp, const T* __restrict__ ru,
                                       const volatile double* pos, int sub, int z0, int zs,
                                       unsigned gmask, double* acc) {
     constexpr int NP = 2 * NB + 2;
-    constexpr int L = tracer_lanes<T>();
     int g[3];
     double fr[3], wx[NP], wy[NP], wz[NP];
 #pragma unroll
@@ -317,16 +341,15 @@ __device__ __forceinline__ void resum(const PParams& pp, const T* __restrict__ r
         for (int d = 0; d < 3; ++d) acc[d] += __shfl_xor_sync(gmask, acc[d], o);
 }
 
-// tracer i of one system, lane `sub` of its pp.split groups of
-// tracer_lanes<T>() lanes (gmask: all of them): gather u(x_i), then (move) the
+// tracer i of one system, lane `sub` of its pp.split groups of L lanes (gmask: all
+// of them; one group where not SPLIT): gather u(x_i), then (move) the
 // Adams-Bashforth step, whose components the first lanes finish.
-template <typename T, int NB, int MM>
+template <typename T, int NB, int MM, int L, bool SPLIT>
 __device__ __forceinline__ void tracer_one(const PParams& pp, const T* __restrict__ ru,
                                            double* __restrict__ pos, double* __restrict__ hist,
                                            double* __restrict__ sample_out, int64_t i, int sub,
                                            unsigned gmask) {
     constexpr int NP = 2 * NB + 2;
-    constexpr int L = tracer_lanes<T>();
     const int N = pp.N;
     double p[3];
     int g[3];
@@ -351,7 +374,7 @@ __device__ __forceinline__ void tracer_one(const PParams& pp, const T* __restric
     }
 
     double acc[3] = {0.0, 0.0, 0.0};
-    const int z0 = tracer_splits<T>(NB) ? sub / L : 0, zs = tracer_splits<T>(NB) ? pp.split : 1;
+    const int z0 = SPLIT ? sub / L : 0, zs = SPLIT ? pp.split : 1;
     row_gather<T, NB, L>(ru, N, g, g[0] - NB, wx, wy, wz, sub % L, z0, zs, gmask, acc[0], acc[1],
                          acc[2]);
     // the groups' planes, pairwise; every lane of the tracer gets the sum
@@ -363,7 +386,7 @@ __device__ __forceinline__ void tracer_one(const PParams& pp, const T* __restric
     // finite is formed again from the stencil's points alone (the sums are the
     // same on all lanes of the tracer, so they all come here together).
     if (!(isfinite(acc[0]) && isfinite(acc[1]) && isfinite(acc[2])))
-        resum<T, NB, MM>(pp, ru, pos + i * 3, sub, z0, zs, gmask, acc);
+        resum<T, NB, MM, L>(pp, ru, pos + i * 3, sub, z0, zs, gmask, acc);
     if (sub >= L) return;
     const size_t slot = (size_t)pp.n * 3;
     const double dt = pp.dt;
@@ -413,26 +436,38 @@ __device__ __forceinline__ void tracer_one(const PParams& pp, const T* __restric
     }
 }
 
-// lanes of one tracer (a power of two)
-template <typename T, int NB>
-__device__ __forceinline__ int tracer_lanes_of(const PParams& pp) {
-    return tracer_splits<T>(NB) ? tracer_lanes<T>() * pp.split : tracer_lanes<T>();
-}
-// lanes of the calling thread's tracer (LR of them), as a shuffle mask
-__device__ __forceinline__ unsigned tracer_group_mask(int LR) {
-    const int lane = threadIdx.x & 31;
-    return (LR == 32 ? 0xffffffffu : (1u << LR) - 1u) << (lane & ~(LR - 1));
+// thread t of a system's blocks: its tracer and lane, in the form that the system
+// takes (LR lanes of one tracer, a power of two; all of them leave together)
+template <typename T, int NB, int MM>
+__device__ __forceinline__ void tracer_thread(const PParams& pp, const T* __restrict__ ru,
+                                              double* __restrict__ pos, double* __restrict__ hist,
+                                              double* __restrict__ sample_out, int64_t t) {
+    auto form = [&](auto lanes, auto split) {
+        constexpr int L = decltype(lanes)::value;
+        constexpr bool SPLIT = decltype(split)::value;
+        const int LR = SPLIT ? L * pp.split : L;
+        const int64_t i = t >> (__ffs(LR) - 1);
+        if (i >= pp.n) return;
+        const int lane = threadIdx.x & 31;
+        const unsigned gmask = (LR == 32 ? 0xffffffffu : (1u << LR) - 1u) << (lane & ~(LR - 1));
+        tracer_one<T, NB, MM, L, SPLIT>(pp, ru, pos, hist, sample_out, i, (int)t & (LR - 1), gmask);
+    };
+    if constexpr (tracer_many_form<T>(NB)) {
+        if (pp.many) {
+            form(std::integral_constant<int, tracer_lanes<T>(NB, true)>(), std::false_type());
+            return;
+        }
+    }
+    form(std::integral_constant<int, tracer_lanes<T>(NB, false)>(),
+         std::integral_constant<bool, tracer_splits<T>(NB)>());
 }
 
 template <typename T, int NB, int MM>
 __global__ void __launch_bounds__(TRACER_THREADS, tracer_min_blocks<T, NB>())
 tracer_kernel(const PParams pp, const T* __restrict__ ru, double* __restrict__ pos,
               double* __restrict__ hist, double* __restrict__ sample_out) {
-    const int LR = tracer_lanes_of<T, NB>(pp);
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t i = t >> (__ffs(LR) - 1);
-    if (i >= pp.n) return;  // all lanes of a tracer leave together
-    tracer_one<T, NB, MM>(pp, ru, pos, hist, sample_out, i, (int)t & (LR - 1), tracer_group_mask(LR));
+    tracer_thread<T, NB, MM>(pp, ru, pos, hist, sample_out,
+                             (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // the tracer systems of many ensemble members in one launch
@@ -482,12 +517,8 @@ tracer_batch_kernel(const TracerSet* __restrict__ sets, const int64_t* __restric
         for (int w = threadIdx.x; w < (int)(sizeof(TracerSet) / 4); w += blockDim.x) dst[w] = src[w];
     }
     __syncthreads();
-    const int LR = tracer_lanes_of<T, NB>(s.pp);
-    const int64_t t = ((int64_t)blockIdx.x - bstart[s_k]) * blockDim.x + threadIdx.x;
-    const int64_t i = t >> (__ffs(LR) - 1);
-    if (i >= s.pp.n) return;  // all lanes of a tracer leave together
-    tracer_one<T, NB, MM>(s.pp, (const T*)s.ru, s.pos, s.hist, nullptr, i, (int)t & (LR - 1),
-                          tracer_group_mask(LR));
+    tracer_thread<T, NB, MM>(s.pp, (const T*)s.ru, s.pos, s.hist, nullptr,
+                             ((int64_t)blockIdx.x - bstart[s_k]) * blockDim.x + threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------

@@ -1,6 +1,6 @@
 """Lanes and lane groups of the tracer gather: tracer counts on both sides of
-every change of the split (tracer_split: 4 lanes a row and up to 37888 threads in
-FP64, 2 lanes in FP32), all stencil widths, stencils across the periodic
+every change of the split (tracer_split: up to 37888 threads; 4 lanes a row in
+FP64, 2 in FP32 and for n = 1) and of the form for many, all stencil widths, stencils across the periodic
 boundary at every lane, values beside a stencil, against the oracle; the same
 bits alone and batched."""
 import numpy as np
@@ -35,7 +35,9 @@ def flow():
 @pytest.mark.parametrize("precision", ["double", "single"])
 @pytest.mark.parametrize("nm,count", [((1, 1), 1), ((1, 0), 2368), ((1, 2), 2369), ((2, 0), 33), ((2, 2), 1184),
                                       ((2, 1), 1185), ((3, 2), 1184), ((3, 0), 4737), ((4, 1), 2369),
-                                      ((4, 0), 4736), ((5, 2), 65), ((5, 1), 9473)])
+                                      ((4, 0), 4736), ((5, 2), 65), ((5, 1), 9473),
+                                      ((1, 1), 4736), ((1, 0), 9472), ((1, 2), 131072), ((1, 2), 131073),
+                                      ((2, 0), 131072), ((2, 0), 131073)])
 def test_sample_at_split_edges(flow, precision, nm, count):
     from bfps_b200.solver import vorticity_equation, particles_system
     w0, ur = flow
@@ -89,17 +91,17 @@ def test_values_beside_the_stencil_do_not_enter(flow, precision, nm, count, bad)
     ve.close()
 
 
-@pytest.mark.parametrize("precision", ["double", "single"])
-def test_batched_systems_of_unequal_split(flow, precision):
+@pytest.mark.parametrize("precision,n", [("double", 2), ("single", 2), ("single", 1)])
+def test_batched_systems_of_unequal_split(flow, precision, n):
     from bfps_b200.solver import NSVEparticles_step, ensemble, particles_system, vorticity_equation
     w0, _ = flow
-    counts = [1, 7, 1184, 1185, 3000, 9473]
+    counts = [1, 7, 1184, 1185, 3000, 9473, 131073]
     ens, a, b = ensemble(), [], []
     for i, c in enumerate(counts):
         for group in (a, b):
             ve = vorticity_equation(N, precision=precision)
             ve.set_cvorticity(w0)
-            group.append((ve, particles_system(ve, _positions(c, i), 2, 0, nsteps=3)))
+            group.append((ve, particles_system(ve, _positions(c, i), n, 0, nsteps=3)))
         ens.add(b[-1][0], 0.01, b[-1][1])
     ens.step(4)
     for (ve, ps), (ve2, ps2) in zip(a, b):
