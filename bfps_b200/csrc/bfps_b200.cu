@@ -214,24 +214,33 @@ static void launch(bool early, void (*kern)(KA...), dim3 grid, int block, size_t
 
 static bool is_pow2(int v) { return v > 0 && (v & (v - 1)) == 0; }
 
-// A kernel whose bounded wait on its own bulk copies ran out sets
-// g_bfg_wait_status (bulk.cuh); read (and cleared) after the work is done.
+// Waits for the context's stream and reads (and clears) the word that a kernel
+// sets whose bounded wait on its own bulk copies ran out (g_bfg_wait_status,
+// bulk.cuh).  The copies go through the context's own non-blocking stream: a
+// copy by cudaMemcpyFromSymbol would wait for everything the caller has queued
+// on its blocking streams, and fail beside another thread's stream capture.
 static int check_wait_status(bfg_ctx* c) {
     int st = 0;
-    CU(cudaMemcpyFromSymbol(&st, g_bfg_wait_status, sizeof(int)));
+    CU(cudaMemcpyFromSymbolAsync(&st, g_bfg_wait_status, sizeof(int), 0, cudaMemcpyDeviceToHost,
+                                 c->stream));
+    CU(cudaStreamSynchronize(c->stream));
     if (st) {
         const int zero = 0;
-        CU(cudaMemcpyToSymbol(g_bfg_wait_status, &zero, sizeof(int)));
+        CU(cudaMemcpyToSymbolAsync(g_bfg_wait_status, &zero, sizeof(int), 0, cudaMemcpyHostToDevice,
+                                   c->stream));
+        CU(cudaStreamSynchronize(c->stream));
         return fail(c, BFG_ECUDA, "a kernel's wait for its own bulk copies ran out");
     }
     return 0;
 }
 
-// end of a call whose result is complete on return: wait, and in FP32 (whose
-// row passes wait for bulk copies) look at the status word
+// end of a call whose result is complete on return: wait, and where the row
+// passes wait for bulk copies (FP32, xpass.cuh and xrows.cuh) look at the status
+// word
 static int finish_call(bfg_ctx* c) {
+    if (c->real_bytes == 4 && c->n >= 64 && c->n <= 512) return check_wait_status(c);
     CU(cudaStreamSynchronize(c->stream));
-    return c->real_bytes == 4 ? check_wait_status(c) : 0;
+    return 0;
 }
 
 static KParams kparams(const bfg_ctx* c, double dt) {
@@ -1340,7 +1349,6 @@ static int field_copy(bfg_ctx* c, int field_id, void* host, bool upload) {
         CU(cudaGetLastError());
         CU(cudaMemcpyAsync(host, c->wb, rows * hpitch, cudaMemcpyDeviceToHost, c->stream));
     }
-    CU(cudaStreamSynchronize(c->stream));
     return check_wait_status(c);
 }
 
@@ -1913,7 +1921,7 @@ int bfg_particles_sample_acceleration(bfg_pctx* p, double* out) {
                             : tracers_dispatch<double>(c, pp, p, p->sample, c->stream, c->v2);
     if (rc) return rc;
     if ((rc = fetch_index_order(p, p->sample, 3, out))) return rc;
-    return c->real_bytes == 4 ? check_wait_status(c) : 0;
+    return finish_call(c);
 }
 
 int bfg_particles_download(bfg_pctx* p, double* pos, double* rhs, int64_t* idx) {
