@@ -66,10 +66,11 @@ struct bfg_ctx {
     std::vector<unsigned char> hmember;  // last uploaded copy
     void* stats_ws = nullptr;  // statistics partial sums
     int* tctr = nullptr;       // 16 words: tile counters of the persistent passes (0, 1:
-                               // self-resetting), outside_scan's result (8)
+                               // self-resetting), upload_state's result (8)
     // what the passes leave out (passes.cuh, modes outside kM): kx columns and
     // the bound on |ky| that may hold modes inside; w0_full: the state may hold
     // modes outside (an upload that did, until it is replaced or low-passed)
+    bool prunes = false;       // the grid's passes leave something out (can_prune)
     int pcols = 0, prow = 0;
     bool w0_full = false;
     unsigned long long* dcount = nullptr;  // bfg_check_finite's counter
@@ -787,6 +788,7 @@ struct OpStep {
 template <typename T, int N>
 struct OpPrune {
     static int run(bfg_ctx* c) {
+        c->prunes = can_prune<T, N>();
         c->pcols = can_prune<T, N>() ? prune_cols(c->kM2, c->dkx, N, col_pblk<T, N>()) : N / 2 + 1;
         c->prow = std::max(prune_k(c->kM2, c->kM2, c->dky, N), 0);
         return 0;
@@ -1126,24 +1128,30 @@ int OpStep<T, N>::run(bfg_ctx* c, double dt, bfg_pctx* p) {
     return E::finish_step(c, E::self(c), 1);
 }
 
-// sets *found where a state-layout field holds a value other than zero at a mode
-// outside kM (one warp per row; the modes inside are not read)
+// pitch_copy8 of an uploaded state into the device rows; sets *found where it
+// holds a value other than zero at a mode outside kM
 template <typename T>
-__global__ void outside_scan(const KParams kp, const cpx<T>* __restrict__ w, int N,
+__global__ void upload_state(const KParams kp, const uint2* __restrict__ src, size_t sq,
+                             uint2* __restrict__ dst, size_t dq, int wq, int N,
                              int* __restrict__ found) {
-    const int lane = threadIdx.x & 31;
-    const int nw = gridDim.x * (blockDim.x >> 5);
     bool any = false;
-    for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < N * N; r += nw) {
+    for (int r = blockIdx.x; r < N * N; r += gridDim.x) {
         const int iy = r / N, iz = r - iy * N;
         const double ky = kp.dky * (double)(iy <= N / 2 ? iy : iy - N);
         const double kz = kp.dkz * (double)(iz <= N / 2 ? iz : iz - N);
-        for (int ix = lane; ix < kp.nxv; ix += 32) {
-            const double kx = ix * kp.dkx;
-            if ((kx * kx + ky * ky) + kz * kz <= kp.kM2) continue;
-            const cpx<T>* a = w + ((size_t)r * kp.nxp + ix) * 3;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) any = any || a[c].x != (T)0 || a[c].y != (T)0;
+        for (int k = threadIdx.x; k < wq; k += blockDim.x) {
+            const uint2 v = src[(size_t)r * sq + k];
+            dst[(size_t)r * dq + k] = v;
+            // a word is one complex number in FP32, half of one in FP64
+            bool set;
+            if constexpr (sizeof(T) == 4)
+                set = __uint_as_float(v.x) != 0.f || __uint_as_float(v.y) != 0.f;
+            else
+                set = __hiloint2double((int)v.y, (int)v.x) != 0.0;
+            if (set) {
+                const double kx = (double)(k * 4 / ((int)sizeof(T) * 3)) * kp.dkx;
+                any = any || !((kx * kx + ky * ky) + kz * kz <= kp.kM2);
+            }
         }
     }
     if (any) *found = 1;
@@ -1324,25 +1332,30 @@ static int field_copy(bfg_ctx* c, int field_id, void* host, bool upload) {
     const int wq = (int)(width / 8);
     if (upload) {
         CU(cudaMemcpyAsync(c->wb, host, rows * hpitch, cudaMemcpyHostToDevice, c->stream));
-        pitch_copy8<<<grid, 256, 0, c->stream>>>((const uint2*)c->wb, hpitch / 8, (uint2*)dev,
-                                                 dpitch / 8, wq, 0, rows);
-        CU(cudaGetLastError());
-        if (field_id == BFG_FIELD_VORTICITY) {
+        if (field_id == BFG_FIELD_VORTICITY && c->prunes) {
+            // looked at while it is copied (128^3 FP32 from pinned memory: 520 us; a
+            // scan of its own and another wait for its result took 535)
             int* found = c->tctr + 8;
             int h = 1;
             c->w0_full = true;
             CU(cudaMemsetAsync(found, 0, sizeof(int), c->stream));
             if (c->real_bytes == 4)
-                outside_scan<float><<<grid, 256, 0, c->stream>>>(kparams(c, 0.0), (const cpx<float>*)dev,
-                                                                 c->n, found);
+                upload_state<float><<<grid, 256, 0, c->stream>>>(
+                    kparams(c, 0.0), (const uint2*)c->wb, hpitch / 8, (uint2*)dev, dpitch / 8, wq, c->n,
+                    found);
             else
-                outside_scan<double><<<grid, 256, 0, c->stream>>>(kparams(c, 0.0),
-                                                                  (const cpx<double>*)dev, c->n, found);
+                upload_state<double><<<grid, 256, 0, c->stream>>>(
+                    kparams(c, 0.0), (const uint2*)c->wb, hpitch / 8, (uint2*)dev, dpitch / 8, wq, c->n,
+                    found);
             CU(cudaGetLastError());
             CU(cudaMemcpyAsync(&h, found, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-            CU(cudaStreamSynchronize(c->stream));
+            if (int rc = check_wait_status(c)) return rc;
             c->w0_full = h != 0;
+            return 0;
         }
+        pitch_copy8<<<grid, 256, 0, c->stream>>>((const uint2*)c->wb, hpitch / 8, (uint2*)dev,
+                                                 dpitch / 8, wq, 0, rows);
+        CU(cudaGetLastError());
     } else {
         pitch_copy8<<<grid, 256, 0, c->stream>>>((const uint2*)dev, dpitch / 8, (uint2*)c->wb,
                                                  hpitch / 8, wq, (int)((hpitch - width) / 8), rows);

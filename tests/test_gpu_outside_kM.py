@@ -100,6 +100,35 @@ def test_single_precision_and_replaced_states(dealias):
 
 
 @pytest.mark.parametrize("precision", ["single", "double"])
+@pytest.mark.parametrize("dealias", [O.SMOOTH, O.TWO_THIRDS])
+def test_upload_sees_single_values_outside(precision, dealias):
+    """One value just outside kM (either part of any component, first and last
+    rows and columns) is kept by a step, but for its part along k; a negative zero
+    there is no value."""
+    dk = (1.0, 1.0, 1.0)
+    ve, ref = _solver(dk, dealias, precision)
+    base = _field(5, dk, dealias, False).astype(ve.cdtype)
+    K2, kM2 = ref.kk.K2, ref.kk.kM2
+    m = int(np.sqrt(kM2))
+    spots = [(0, 0, m + 1), (0, m + 1, 1), (N - 1, 0, m + 1), (N // 2, N // 2, N // 2), (N - m - 1, 0, 1),
+             (m + 1, N - 1, 2)]
+    for i, at in enumerate(spots):
+        assert K2[at] > kM2
+        k = np.array([at[2]] + [j if j <= N // 2 else j - N for j in at[:2]], float)
+        for value in ((1e-3, 1e-3j)[i % 2], complex(-0.0, -0.0)):
+            w = base.copy()
+            w[at][(i + 1) % 3] = value
+            ve.set_cvorticity(w)
+            ve.step(1e-3)
+            got = ve.get_cvorticity()
+            want = w[at] - k * (k @ w[at]) / (k @ k)
+            assert np.abs(got[at] - want).max() <= 1e-5 * abs(value), (at, value)
+            got[at] = 0
+            assert not got[K2 > kM2].any(), (at, value)
+    ve.close()
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
 def test_ensemble_of_unequal_members(precision):
     """Members with different rules, boxes and states (one full, replaced while
     in the ensemble): bit-identical to stepping alone."""
