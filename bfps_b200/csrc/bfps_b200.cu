@@ -287,21 +287,36 @@ static double kwrap_h(int i, int N, double dk) { return dk * (double)(i <= N / 2
 
 // --------------------------------------------------------- autotuning --
 // Column-pass schedule (passes.cuh: 0 or 1) per (device, grid size, real
-// bytes, pass kind, members per launch).  The member count is part of the key
-// because the better schedule depends on how many tiles one launch holds: a
+// bytes, pass kind, members per launch, tiles).  The member count is part of the
+// key because the better schedule depends on how many tiles one launch holds: a
 // lone 64^3 context and a group of sixteen 64^3 ensemble members choose
-// differently.  Filled by bfg_autotune (one member), bfg_ens_autotune (each
-// size group of an ensemble), bfg_tune_set and, where the environment
-// variable BFPS_B200_TUNE_CACHE names a file, by the choices recorded there
-// by earlier runs on a device of the same name (one line per choice: device
-// name, N, real bytes, pass kind, members, schedule, and the two measured
-// times in ms).  Entries not tuned for that exact key use schedule 0.
+// differently.  So is what the passes leave out of a grid (the kx columns and
+// the bound on |ky| that they keep; 0, 0 where they keep all): the smooth filter
+// and the two-thirds rule leave 79 % and 35 % of the columns.  Filled by
+// bfg_autotune (one member), bfg_ens_autotune (each size group of an ensemble) and,
+// where the environment variable BFPS_B200_TUNE_CACHE names a file, by the
+// choices recorded there by earlier runs on a device of the same name (one line
+// per choice: device name, N, real bytes, pass kind, members, schedule, the two
+// measured times in ms, kx columns, |ky| bound; lines without the last two were
+// measured on whole grids and hold for those).  bfg_tune_set imposes a schedule
+// whatever is left out.  Entries not tuned for that exact key use schedule 0.
+// (A state with modes outside kM runs its first inverse passes and the last
+// forward one whole; the choice is the one of the other stages.)
 struct TuneEntry {
     int sched = 0;
     double ms0 = 0, ms1 = 0;
 };
 static std::mutex g_tune_mu;
-using TuneKey = std::tuple<int, int, int, int, int>;  // device, N, real bytes, kind, members
+// device, N, real bytes, kind, members, kx columns, |ky| bound
+using TuneKey = std::tuple<int, int, int, int, int, int, int>;
+static TuneKey tune_key(const bfg_ctx* c, int kind, int members) {
+    return TuneKey(c->device, c->n, c->real_bytes, kind, members, c->prunes ? c->pcols : 0,
+                   c->prunes ? c->prow : 0);
+}
+// bfg_tune_set's entry: any tiles
+static TuneKey tune_any(const bfg_ctx* c, int kind, int members) {
+    return TuneKey(c->device, c->n, c->real_bytes, kind, members, -1, -1);
+}
 static std::map<TuneKey, TuneEntry> g_tune;
 static std::map<int, bool> g_tune_loaded;  // device -> cache file read
 
@@ -331,24 +346,32 @@ static void tune_load_locked(int dev) {
     FILE* f = std::fopen(path, "r");
     if (!f) return;
     const std::string me = device_name(dev);
-    char name[256];
-    int n, rb, kind, nmem, sched;
+    char line[512], name[256];
+    int n, rb, kind, nmem, sched, pcols, prow;
     double ms0, ms1;
-    while (std::fscanf(f, "%255s %d %d %d %d %d %lf %lf", name, &n, &rb, &kind, &nmem, &sched, &ms0,
-                       &ms1) == 8)
-        if (me == name && (sched == 0 || sched == 1) && nmem >= 1) {
-            TuneEntry& e = g_tune[TuneKey(dev, n, rb, kind, nmem)];
+    while (std::fgets(line, sizeof(line), f)) {
+        const int got = std::sscanf(line, "%255s %d %d %d %d %d %lf %lf %d %d", name, &n, &rb, &kind, &nmem,
+                                    &sched, &ms0, &ms1, &pcols, &prow);
+        if (got == 8) pcols = prow = 0;
+        if ((got == 8 || got == 10) && me == name && (sched == 0 || sched == 1) && nmem >= 1) {
+            TuneEntry& e = g_tune[TuneKey(dev, n, rb, kind, nmem, pcols, prow)];
             e.sched = sched;
             e.ms0 = ms0;
             e.ms1 = ms1;
         }
+    }
     std::fclose(f);
 }
-static int tuned_schedule(int dev, int n, int rb, int kind, int nmem) {
+// the entry for a launch of `members` members as c runs it (g_tune_mu held)
+static TuneEntry tune_find_locked(const bfg_ctx* c, int kind, int members) {
+    tune_load_locked(c->device);
+    auto it = g_tune.find(tune_key(c, kind, members));
+    if (it == g_tune.end()) it = g_tune.find(tune_any(c, kind, members));
+    return it == g_tune.end() ? TuneEntry() : it->second;
+}
+static int tuned_schedule(const bfg_ctx* c, int kind, int members) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    tune_load_locked(dev);
-    auto it = g_tune.find(TuneKey(dev, n, rb, kind, nmem));
-    return it == g_tune.end() ? 0 : it->second.sched;
+    return tune_find_locked(c, kind, members).sched;
 }
 // Schedule 1 replaces the default only when it is faster by more than a
 // margin: the tuner times one launch at a time, and schedule 0 (two CTAs per
@@ -362,23 +385,23 @@ constexpr double TUNE_MARGIN = 0.02;
 constexpr double TUNE_MARGIN_SHARED = 0.10;
 
 // record measured times (ms[kind * 2 + schedule]) for nmem members per
-// launch, the chosen schedule, and append them to the cache file
-static void tune_store(int dev, int n, int rb, int nmem, const double* ms,
-                       double margin = TUNE_MARGIN) {
+// launch as c runs them, the chosen schedule, and append them to the cache file
+static void tune_store(const bfg_ctx* c, int nmem, const double* ms, double margin = TUNE_MARGIN) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    tune_load_locked(dev);
+    tune_load_locked(c->device);
     const char* path = std::getenv("BFPS_B200_TUNE_CACHE");
     FILE* f = (path && *path) ? std::fopen(path, "a") : nullptr;
-    const std::string name = device_name(dev);
+    const std::string name = device_name(c->device);
     for (int kind : {(int)K_IZ, (int)K_IY, (int)K_FY, (int)K_FZ}) {
         TuneEntry e;
         e.ms0 = ms[2 * kind];
         e.ms1 = ms[2 * kind + 1];
         e.sched = e.ms1 < e.ms0 * (1.0 - margin) ? 1 : 0;
-        g_tune[TuneKey(dev, n, rb, kind, nmem)] = e;
+        const TuneKey key = tune_key(c, kind, nmem);
+        g_tune[key] = e;
         if (f)
-            std::fprintf(f, "%s %d %d %d %d %d %.6f %.6f\n", name.c_str(), n, rb, kind, nmem, e.sched,
-                         e.ms0, e.ms1);
+            std::fprintf(f, "%s %d %d %d %d %d %.6f %.6f %d %d\n", name.c_str(), c->n, c->real_bytes, kind,
+                         nmem, e.sched, e.ms0, e.ms1, std::get<5>(key), std::get<6>(key));
     }
     if (f) std::fclose(f);
 }
@@ -398,7 +421,7 @@ struct Engine {
     // member count
     template <int MODE>
     static int col(bfg_ctx* c, const Mem* mem, int nmem, Roles rl) {
-        return tuned_schedule(c->device, N, (int)sizeof(T), col_kind(MODE), nmem) == 1
+        return tuned_schedule(c, col_kind(MODE), nmem) == 1
                    ? col_s<MODE, 1>(c, mem, nmem, rl)
                    : col_s<MODE, 0>(c, mem, nmem, rl);
     }
@@ -1757,16 +1780,14 @@ int bfg_autotune(bfg_ctx* c, int reps) {
     if ((rc = sync_member(c, dt))) return rc;
     double ms[2 * BFG_NKINDS] = {0};
     if ((rc = dispatch<OpTune>(c, reps, ms))) return rc;
-    tune_store(c->device, c->n, c->real_bytes, 1, ms);
+    tune_store(c, 1, ms);
     return 0;
 }
 
 int bfg_tune_get(const bfg_ctx* c, int kind, int members, int* schedule, double* ms0, double* ms1) {
     if (!c || !col_kind_valid(kind) || members < 1) return BFG_EINVAL;
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    tune_load_locked(c->device);
-    auto it = g_tune.find(TuneKey(c->device, c->n, c->real_bytes, kind, members));
-    const TuneEntry e = it == g_tune.end() ? TuneEntry() : it->second;
+    const TuneEntry e = tune_find_locked(c, kind, members);
     if (schedule) *schedule = e.sched;
     if (ms0) *ms0 = e.ms0;
     if (ms1) *ms1 = e.ms1;
@@ -1778,7 +1799,15 @@ int bfg_tune_set(bfg_ctx* c, int kind, int members, int schedule) {
         return BFG_EINVAL;
     std::lock_guard<std::mutex> lk(g_tune_mu);
     tune_load_locked(c->device);
-    g_tune[TuneKey(c->device, c->n, c->real_bytes, kind, members)].sched = schedule;
+    const TuneKey any = tune_any(c, kind, members);
+    g_tune[any].sched = schedule;
+    // and over what was measured for any tiles
+    for (auto it = g_tune.lower_bound(any); it != g_tune.end(); ++it) {
+        TuneKey k = it->first;
+        std::get<5>(k) = std::get<6>(k) = -1;
+        if (k != any) break;
+        it->second.sched = schedule;
+    }
     return 0;
 }
 
@@ -2311,6 +2340,7 @@ static int ens_prepare(bfg_ens* e) {
         // the launches cover what any member holds
         for (int i : g->members) {
             const bfg_ctx* ci = e->entries[i].ctx;
+            g->launcher.prunes = ci->prunes;  // by size and precision alone
             g->launcher.pcols = std::max(g->launcher.pcols, ci->pcols);
             g->launcher.prow = std::max(g->launcher.prow, ci->prow);
             g->launcher.w0_full = g->launcher.w0_full || ci->w0_full;
@@ -2585,7 +2615,7 @@ int bfg_ens_autotune(bfg_ens* e, int reps) {
         double ms[2 * BFG_NKINDS] = {0};
         rc = e->real_bytes == 4 ? ens_group_tune<float>(g, reps, ms) : ens_group_tune<double>(g, reps, ms);
         if (rc) return ens_fail(e, rc, g->launcher.err.c_str());
-        tune_store(e->device, g->n, e->real_bytes, (int)g->members.size(), ms,
+        tune_store(&g->launcher, (int)g->members.size(), ms,
                    e->groups.size() > 1 ? TUNE_MARGIN_SHARED : TUNE_MARGIN);
     }
     // captured graphs hold the old schedules: rebuild them before the next step

@@ -273,9 +273,10 @@ int bfg_profile_read(bfg_ctx* ctx, int kind, double* total_ms, int64_t* launches
  * 3 FY, 4 FZ) is built in two schedules: 0, two 256-thread CTAs per SM with
  * one tile buffer each and 32-point butterflies in FP32; 1, one 512-thread
  * CTA with two tile buffers and radix-8 butterflies.  The choice is kept per
- * device, grid size, precision and members per launch (1 for a lone
- * context; the size of an ensemble's group of equal grids otherwise), since
- * the better schedule depends on how many tiles one launch holds.
+ * device, grid size, precision, members per launch (1 for a lone context; the
+ * size of an ensemble's group of equal grids otherwise) and what the passes
+ * leave out of the grid (modes outside kM, from 128^3 up), since the better
+ * schedule depends on how many tiles one launch holds.
  * bfg_autotune times both on this context's buffers (reps launches each,
  * after one warm-up; only the work buffers are written, so the complex and
  * real velocity of the context are lost) for one member per launch.
@@ -289,7 +290,7 @@ int bfg_profile_read(bfg_ctx* ctx, int kind, double* total_ms, int64_t* launches
  * and read back by later processes on a device of the same name.  A key
  * never tuned uses schedule 0.  bfg_tune_get reads the choice for a member
  * count and its measured times (0 when not measured), bfg_tune_set imposes
- * one. */
+ * one on every context of the size and precision. */
 int bfg_autotune(bfg_ctx* ctx, int reps);
 int bfg_ens_autotune(bfg_ens* e, int reps);
 int bfg_tune_get(const bfg_ctx* ctx, int kind, int members, int* schedule, double* ms0, double* ms1);

@@ -146,3 +146,46 @@ def test_ensemble_autotune_then_other_schedule_equals_alone(graphs):
             if ps is not None:
                 ps.close()
             ve.close()
+
+
+def test_choice_belongs_to_what_the_passes_leave_out(tmp_path, monkeypatch):
+    """Contexts of one size whose passes keep different modes (smooth filter,
+    two-thirds rule) do not share measured choices; an imposed one holds for
+    both.  Cache lines without the tiles hold for whole grids only."""
+    import subprocess
+    import sys
+    import torch
+    from bfps_b200 import _lib
+    from bfps_b200.solver import vorticity_equation
+    cache = tmp_path / "tune.txt"
+    monkeypatch.setenv("BFPS_B200_TUNE_CACHE", str(cache))
+    smooth = vorticity_equation(128, precision="single", dealias_type=_lib.SMOOTH)
+    thirds = vorticity_equation(128, precision="single", dealias_type=_lib.TWO_THIRDS)
+    try:
+        thirds.autotune(reps=1)
+        assert all(v[1] > 0 and v[2] > 0 for v in thirds.schedules().values())
+        assert all(v == (0, 0.0, 0.0) for v in smooth.schedules().values())
+        times = thirds.schedules()["IZ"][1:]
+        for s in (1, 0):
+            smooth.set_schedule("IZ", s)
+            assert smooth.schedules()["IZ"][0] == s and thirds.schedules()["IZ"] == (s,) + times
+    finally:
+        for p in PASSES:
+            smooth.set_schedule(p, 0)
+        smooth.close()
+        thirds.close()
+    rows = [l.split() for l in cache.read_text().splitlines()]
+    assert len(rows) == 4 and all(len(r) == 10 for r in rows)
+    tiles = " ".join(rows[0][8:])
+    name = torch.cuda.get_device_name().replace(" ", "_")
+    cache.write_text("%s 32 8 0 1 1 0.5 0.25\n%s 128 4 0 1 1 0.5 0.25\n%s 128 4 1 1 1 0.5 0.25 %s\nnot a line\n"
+                     "%s 64 4 0 1 1 0.5 0.25 0 0\n" % (name, name, name, tiles, name))
+    code = ("from bfps_b200 import _lib\nfrom bfps_b200.solver import vorticity_equation as V\n"
+            "print(V(32, precision='double').schedules()['IZ'], V(64, precision='single').schedules()['IZ'])\n"
+            "t = V(128, precision='single', dealias_type=_lib.TWO_THIRDS).schedules()\n"
+            "print(t['IZ'], t['IY'], V(128, precision='single').schedules()['IY'])\n")
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                         cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert out.returncode == 0, out.stderr
+    hit, miss = (1, 0.5, 0.25), (0, 0.0, 0.0)
+    assert out.stdout.split("\n")[:2] == ["%s %s" % (hit, hit), "%s %s %s" % (miss, hit, miss)]
