@@ -1,8 +1,8 @@
 """Lanes and lane groups of the tracer gather: tracer counts on both sides of
 every change of the split (tracer_split: up to 37888 threads; 4 lanes a row in
-FP64, 2 in FP32 and for n = 1) and of the form for many, all stencil widths, stencils across the periodic
-boundary at every lane, values beside a stencil, against the oracle; the same
-bits alone and batched."""
+FP64, 2 in FP32 and for n = 1) and of the form for many, all stencil widths,
+stencils across the periodic boundary at every lane, values beside a stencil,
+against the oracle; the same bits alone and batched."""
 import numpy as np
 import pytest
 
@@ -114,8 +114,9 @@ def test_batched_systems_of_unequal_split(flow, precision, n):
 @pytest.mark.parametrize("n", [16, 32, 64, 128])
 @pytest.mark.parametrize("precision", ["double", "single"])
 def test_launches_that_start_early_see_what_came_before(n, precision):
-    """Passes of small grids are launched while the pass before them drains:
-    steps queued back to back give the bits of steps waited for one by one."""
+    """Passes of small grids are launched while the pass before them drains.  At the
+    end of a step (inside, both sides launch alike): steps queued back to back give
+    the bits of steps waited for one by one."""
     from bfps_b200.solver import NSVEparticles_step, particles_system, vorticity_equation
     out = []
     for wait in (True, False):
