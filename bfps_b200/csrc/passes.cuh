@@ -1356,19 +1356,11 @@ row_nonlin(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __re
     pdl_wait();
     pdl_release();
 
-    // kx columns that the rows of a member hold on each side (read again only
-    // where the member changes)
-    int pm = -1, pc = M + 1;
+    // kx columns that the rows of a member hold on each side (looked up where they
+    // are needed: kept in registers through the phases they cost spills)
     auto cols = [&](int mm, int side) {
-        if constexpr (can_prune<T, N>()) {
-            if (mm != pm) {
-                pm = mm;
-                pc = mem[mm].kp.pcols;
-            }
-            return rl.prune & side ? pc : M + 1;
-        } else {
-            return M + 1;
-        }
+        if constexpr (can_prune<T, N>()) return rl.prune & side ? mem[mm].kp.pcols : M + 1;
+        else return M + 1;
     };
     auto issue = [&](int tt) {
         const int mm = tt / tiles_per, tl = tt - mm * tiles_per;
@@ -1381,14 +1373,18 @@ row_nonlin(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __re
                 const int v = e - b * NV;
                 cp_async16(&st[b * ROWS * RL + v * VPE], &(b ? sw : su)[v * VPE]);
             }
-        } else {  // the rows' first kin columns, zeros after them
-            constexpr int RV = RL / VPE;
-            for (int e = tid; e < 2 * NV; e += RNL_THREADS) {
-                const int b = e >= NV ? 1 : 0;
-                const int v = e - b * NV;
-                cpx<T>* dst = &st[b * ROWS * RL + v * VPE];
-                if ((v % RV) * VPE < kin * 3) cp_async16(dst, &(b ? sw : su)[v * VPE]);
-                else *reinterpret_cast<float4*>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {
+            // the rows' first kin columns, a warp per row; the zeros after them stay
+            // in the staging rows, which nothing else writes, until a member that
+            // keeps another number of columns
+            const bool fill = tt < (int)gridDim.x || cols((tt - (int)gridDim.x) / tiles_per, PRUNE_IN) != kin;
+            static_assert(!can_prune<T, N>() || col_pblk<T, N>() * 3 % VPE == 0, "whole vectors");
+            const int nv = kin * 3 / VPE;
+            for (int r = tid >> 5; r < 2 * ROWS; r += RNL_THREADS / 32) {
+                const cpx<T>* src = r < ROWS ? su + r * RL : sw + (r - ROWS) * RL;
+                for (int v = tid & 31; v < nv; v += 32) cp_async16(&st[r * RL + v * VPE], &src[v * VPE]);
+                if (fill)
+                    for (int v = nv * VPE + (tid & 31); v < RL; v += 32) st[r * RL + v] = zero_c<T>();
             }
         }
     };
@@ -1400,7 +1396,6 @@ row_nonlin(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __re
         __syncthreads();
         const int m = t / tiles_per, tl = t - m * tiles_per;
         const size_t row0 = (size_t)tl * ROWS;
-        const int kin = cols(m, PRUNE_IN), kout = cols(m, PRUNE_OUT);
 
         // A: C2R pre-processing + DIF stage 0, staging rows -> pencils
         for (int e = tid; e < 6 * ROWS * H0; e += RNL_THREADS) {
@@ -1431,7 +1426,7 @@ row_nonlin(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __re
                 }
             } else {
                 // item 0: k = S0 q pairs with S0 (R0 - q); X[0] with X[M]
-                const T x0 = va[0].x, xm = M < kin ? x[3 * M].x : (T)0;
+                const T x0 = va[0].x, xm = M < cols(m, PRUNE_IN) ? x[3 * M].x : (T)0;
                 va[0] = mk<T>(x0 + xm, x0 - xm);
 #pragma unroll
                 for (int q = 1; q < R0 / 2; ++q) {
@@ -1645,6 +1640,7 @@ row_nonlin(const Member<T>* __restrict__ mem, const Roles rl, const cpx<T>* __re
         {
             cpx<T>* wout = mbuf(mem[m], rl.out0) + row0 * RL;
             float4* dst = reinterpret_cast<float4*>(wout);
+            const int kout = cols(m, PRUNE_OUT);
             for (int v = tid; v < NV; v += RNL_THREADS) {
                 const int r = v / (RL / VPE);
                 if (kout < M && (v - r * (RL / VPE)) * VPE >= kout * 3) continue;
