@@ -65,6 +65,16 @@ def peaks():
         return 6650.0, "fallback"
 
 
+def kept_fractions(cfg):
+    """s, d, x: what the passes keep of a field in the state layout, between the
+    z and y passes, and around the x pass (modes inside kM; 1 below 128^3)."""
+    n = cfg["n"]
+    if n < 128:
+        return 1.0, 1.0, 1.0
+    x = (n // 2 - 1 if cfg["dealias"] == 1 else n // 3 - 1) / (n / 2)
+    return math.pi / 6 * x ** 3, math.pi / 4 * x ** 2, x
+
+
 def algorithmic_bytes(cfg):
     """Per-step and per-kernel-launch algorithmic bytes.
 
@@ -86,10 +96,7 @@ def algorithmic_bytes(cfg):
     nt = cfg["ntracers"]
     real3 = 3 * n ** 3 * P
     step = 105 * U + nt * 24 * (k + 2) + 2 * real3
-    x = d = s = 1.0
-    if n >= 128:
-        x = (n // 2 - 1 if cfg["dealias"] == 1 else n // 3 - 1) / (n / 2)
-        d, s = math.pi / 4 * x ** 2, math.pi / 6 * x ** 3
+    s, d, x = kept_fractions(cfg)
     per_launch = {
         "IZ": (3 * s + 6 * d) * U,
         "IY": (6 * d + 6 * x) * U,
@@ -105,9 +112,16 @@ def algorithmic_bytes(cfg):
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of one launch
 # divided by its algorithmic bytes, from the ncu captures summarised under
-# profiles/ (256^3 FP32 stage 1 passes; tracer kernel at 4e6 tracers on 256^3).
-# Traffic at another size is taken to scale with the algorithmic bytes.
-TRAFFIC_RATIO = {"X": 0.954, "IZ": 0.953, "IY": 0.972, "FY": 0.896, "FZ": 1.03, "tracers": 0.983}
+# profiles/ (256^3 FP32 passes with the smooth filter; tracer kernel at 4e6
+# tracers on 256^3).  Traffic at another size from 128^3 up is taken to scale with
+# the algorithmic bytes; it is not given for the two-thirds rule or smaller grids,
+# nor for FZ, which was captured in stage 1 only (1.03) while the line's figure is
+# the average of the stages.
+TRAFFIC_RATIO = {"X": 0.954, "IZ": 0.953, "IY": 0.972, "FY": 0.896, "tracers": 0.983}
+
+
+def traffic_ratio(cfg, kernel):
+    return TRAFFIC_RATIO.get(kernel) if cfg["n"] >= 128 and cfg["dealias"] == 1 else None
 
 
 class ClockSampler:
@@ -220,10 +234,12 @@ def acceleration_report(ve, ps, cfg, reps=3):
     """NSVEparticles::do_stats acceleration sampling (pressure, Lagrangian
     acceleration, inverse transform, tracer gather) on the current state:
     device time per call from per-launch CUDA events, and achieved bandwidth
-    against its algorithmic bytes, 109 U + 48 n (19 launches: velocity to
-    real space 18U, two products 12U, two forward transforms 36U, two
-    pressure contractions 9U, velocity 6U, acceleration 7U, inverse
-    transform 18U, gather 3U + 48 n)."""
+    against its algorithmic bytes (s, d, x as in kept_fractions): velocity to
+    real space (3 + 3s + 6d + 6x)U, two forward transforms 36U, two pressure
+    contractions (7 + 2s)U, velocity (3 + 3s)U, acceleration (3 + 4s)U, inverse
+    transform (3 + 3s + 6d + 6x)U, gather 3U + 48 n: 18 launches in FP32 from 64^3
+    to 512^3, where the row kernel forms the products; elsewhere two kernels
+    more that write and read them, 12U."""
     from bfps_b200 import _lib
     L = _lib.lib()
     out = np.empty((ps.n, 3))
@@ -241,7 +257,9 @@ def acceleration_report(ve, ps, cfg, reps=3):
     ms = tot / reps
     P = 4 if cfg["precision"] == "single" else 8
     U = cfg["n"] ** 2 * (cfg["n"] + 2) * P
-    nbytes = 109 * U + 48 * ps.n
+    s, d, x = kept_fractions(cfg)
+    fused = cfg["precision"] == "single" and 64 <= cfg["n"] <= 512
+    nbytes = (58 + 15 * s + 12 * d + 12 * x + (0 if fused else 12)) * U + 48 * ps.n
     peak, _ = peaks()
     return {"device_ms": round(ms, 3), "launches_per_call": n // reps,
             "algorithmic_bytes": int(nbytes), "achieved_gbs": round(nbytes / (ms / 1e3) / 1e9, 1),
@@ -374,8 +392,8 @@ def run_ours(args, cfg):
         ach = per_launch[dominant] / (avg / 1e3) / 1e9
         roof = {"bound": "hbm", "kernel": dominant, "achieved": round(ach, 1), "peak": peak,
                 "unit": "GB/s", "frac": round(ach / peak, 4),
-                "traffic": (round(TRAFFIC_RATIO[dominant] * per_launch[dominant])
-                            if dominant in TRAFFIC_RATIO else None),
+                "traffic": (round(traffic_ratio(cfg, dominant) * per_launch[dominant])
+                            if traffic_ratio(cfg, dominant) else None),
                 "traffic_source": "ncu dram bytes per launch / algorithmic bytes (profiles/), "
                                   "scaled to this size",
                 "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else peak_kind}

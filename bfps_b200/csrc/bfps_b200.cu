@@ -191,10 +191,12 @@ struct Prof {
 // Launch of a pass that may be scheduled while the launch before it on the
 // stream drains (programmatic dependent launch; every such kernel calls
 // pdl_wait() before it touches anything an earlier launch may write, fft.cuh).
-// `early` for short launches only, whose start-up shows: a step at 32^3 FP64 takes
-// 98 us instead of 138, at 64^3 FP32 170 instead of 206, at 128^3 FP64 755 instead
-// of 796; at 256^3 FP32, where the x pass's one block per SM comes up unevenly, it
-// lost (2461 against 2373 us), and so did a mixed ensemble with it everywhere.
+// `early` for launches of up to 2^22 grid points only, whose start-up shows (a
+// step, waiting / early): 64^3 FP32 200 / 162 us, FP64 213 / 190, 128^3 FP32 430 /
+// 405, FP64 729 / 700; 32^3 FP64 with tracers 138 / 98.  Above, nothing is gained in
+// FP64 (256^3 4440 / 4436, two-thirds rule 3110 / 3116), and FP32, where the x
+// pass's one block per SM comes up unevenly, loses (256^3 2270 / 2380, two-thirds
+// rule 1541 / 1643), as did a mixed ensemble.
 template <typename... KA, typename... A>
 static void launch(bool early, void (*kern)(KA...), dim3 grid, int block, size_t smem, cudaStream_t st,
                    A... args) {
@@ -1623,7 +1625,8 @@ int bfg_field_stats(bfg_ctx* c, const void* field, double max_estimate, int nbin
     if (int ro = order_after_caller(c, field, nullptr)) return ro;
     int rc = sync_member(c, c->fac_dt);
     if (rc) return rc;
-    // into v1 (free between steps), re-pitched to the device rows
+    // into v1 (not needed between steps: stats_engine.inl), re-pitched to the
+    // device rows
     const size_t N = c->n, cb = 2 * (size_t)c->real_bytes;
     CU(cudaMemset2DAsync(c->v1, c->nxp * 3 * cb, 0, c->nxp * 3 * cb, N * N, c->stream));
     CU(cudaMemcpy2DAsync(c->v1, c->nxp * 3 * cb, field, c->nxv * 3 * cb, c->nxv * 3 * cb, N * N,

@@ -1,7 +1,10 @@
 // Engine<T, N>::stats — field::compute_stats (bfps/cpp/field.cpp:984-1040)
 // for one complex 3-vector field in the state layout: co-spectrum, then the
-// unnormalised C2R into scratch (v2 is free between steps: every step
-// rewrites it completely) and the real-space moments and histograms.
+// unnormalised C2R into scratch and the real-space moments and histograms.
+// The scratch is v2: between steps nothing in v1 and v2 is needed.  A step writes
+// and reads them inside the region that the passes keep (passes.cuh, modes
+// outside kM) and nowhere else, so what is left here stays in v2 outside it: a
+// pass that reads v1 or v2 has to leave the same modes out (PRUNE_IN).
 // Included by bfps_b200.cu after the Engine definition.
 
 template <typename T, int N>
