@@ -92,7 +92,7 @@ constexpr int TRACER_THREADS = 128;
 // tracers, n = 4, m = 1, 256^3): 490 us with one lane, 250 us with four (190 us
 // with the loop shape below).  Narrow FP64 stencils have few sectors a row, so the
 // lanes' own work weighs more: n = 1, 1e6 tracers, 128^3: 347 us with four lanes,
-// 260 with two; n = 2: 5000 tracers 15 us with four lanes, 21 with two, but 1e6
+// 260 with two; n = 2: 300 tracers 9 us with four lanes, 11 with two, but 1e6
 // in cell order 707 against 610.  So n = 2 takes two for many tracers.
 template <typename T>
 __host__ __device__ constexpr int tracer_lanes(int nb, bool many) {
@@ -142,8 +142,8 @@ __host__ __device__ inline int tracer_many(int64_t n, int nb) {
 //   FP32, n = 3: eight rows, four blocks (4e6 tracers, 512^3: 2.43 ms; five blocks
 //   2.47-2.52, four rows and six blocks 2.57); n = 2: three, four (1e5 tracers,
 //   256^3: 75 us; one and six 100, two and five 94, six rows 76); n = 1: two, six
-//   (1e6, 128^3: 205 us; three and four 234, two and eight 197 but 5000 tracers 12
-//   against 11); n = 4: two, four (1e6, 128^3: 1.68 ms; three and four 1.77, one and
+//   (1e6, 128^3: 205 us; three and four 234, two and eight 197, but 20000 tracers 17
+//   against 15); n = 4: two, four (1e6, 128^3: 1.68 ms; three and four 1.77, one and
 //   four 1.93); n = 5: three, four.
 //   FP64: two rows, and three for n = 2 (1e6, 128^3: 641 us; two 659); four blocks,
 //   n = 1 five (1e6, 128^3: 260 us; four 286).  n = 4, 50001 tracers, 256^3: 190 us;
