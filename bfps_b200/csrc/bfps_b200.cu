@@ -70,6 +70,7 @@ struct bfg_ctx {
     // what the passes leave out (passes.cuh, modes outside kM): kx columns and
     // the bound on |ky| that may hold modes inside; w0_full: the state may hold
     // modes outside (an upload that did, until it is replaced or low-passed)
+    bool captured = false;     // launches go into the graphs of an ensemble of one size
     bool prunes = false;       // the grid's passes leave something out (can_prune)
     int pcols = 0, prow = 0;
     bool w0_full = false;
@@ -191,12 +192,17 @@ struct Prof {
 // Launch of a pass that may be scheduled while the launch before it on the
 // stream drains (programmatic dependent launch; every such kernel calls
 // pdl_wait() before it touches anything an earlier launch may write, fft.cuh).
-// `early` for launches of up to 2^22 grid points only, whose start-up shows (a
-// step, waiting / early): 64^3 FP32 200 / 162 us, FP64 213 / 190, 128^3 FP32 430 /
-// 405, FP64 729 / 700; 32^3 FP64 with tracers 138 / 98.  Above, nothing is gained in
-// FP64 (256^3 4440 / 4436, two-thirds rule 3110 / 3116), and FP32, where the x
-// pass's one block per SM comes up unevenly, loses (256^3 2270 / 2380, two-thirds
-// rule 1541 / 1643), as did a mixed ensemble.
+// `early` for short launches only, whose start-up shows.  On a stream: up to 2^22
+// grid points (a step, waiting / early: 64^3 FP32 200 / 162 us, FP64 213 / 190, 128^3
+// FP32 430 / 405, FP64 729 / 700; 32^3 FP64 with tracers 138 / 98).  Above, nothing
+// is gained in FP64 (256^3 4440 / 4436, two-thirds rule 3110 / 3116), and FP32, where
+// the x pass's one block per SM comes up unevenly, loses (256^3 2270 / 2380,
+// two-thirds rule 1541 / 1643).  In the captured graphs of an ensemble of one
+// size, whose launches have short gaps anyway: up to 2^20 (FP32: 1 x 32^3 76 / 64, 16 x
+// 32^3 160 / 155, 40 x 32^3 334 / 341, 8 x 64^3 442 / 439, 16 x 64^3 841 / 874, 1 x
+// 128^3 395 / 415, 2 x 128^3 719 / 798).  Groups of several sizes run beside each
+// other and fill in for one another: with 2^20 for them a mixed ensemble of 32^3,
+// 64^3 and 128^3 members took 106.5 ms instead of 104.8.
 template <typename... KA, typename... A>
 static void launch(bool early, void (*kern)(KA...), dim3 grid, int block, size_t smem, cudaStream_t st,
                    A... args) {
@@ -414,9 +420,10 @@ struct Engine {
     using C = cpx<T>;
     using Mem = Member<T>;
 
-    // launches of up to 2^22 grid points (a 128^3 grid, sixteen 64^3 members)
-    // may start while the launch before drains: launch()
-    static bool early(int nmem) { return (size_t)N * N * N * nmem <= ((size_t)1 << 22); }
+    // whether a launch may start while the launch before drains: launch()
+    static bool early(const bfg_ctx* c, int nmem) {
+        return (size_t)N * N * N * nmem <= (size_t)1 << (c->captured ? 20 : 22);
+    }
 
     // one persistent launch of a column pass over nmem members, in the
     // schedule the autotuner chose for this grid, precision, pass and
@@ -446,7 +453,12 @@ struct Engine {
         Prof pr(c, col_kind(MODE));
         // dynamic tile order where a launch has at least 8 tiles per CTA
         int* tctr = ntiles >= 8 * grid ? c->tctr : nullptr;
-        launch(early(nmem), kern, grid, col_threads<T, N, MODE, S>(), smem, c->stream, mem, rl, (const C*)c->tw, ntx,
+        // IY over a few 16^3 members waits: as the only early pass it took their step
+        // from 94 to 101 us (8 members, FP32) and from 244 to 280 (32); the others
+        // early without it 91 and 244, all early 99 and 285; one member 45 with it,
+        // 51 without
+        const bool wait = N == 16 && MODE == CM_Y_INV2 && nmem >= 4;
+        launch(early(c, nmem) && !wait, kern, grid, col_threads<T, N, MODE, S>(), smem, c->stream, mem, rl, (const C*)c->tw, ntx,
                kdom, tiles_per, ntiles, tctr);
         return after_launch(c, "col_pass");
     }
@@ -514,7 +526,7 @@ struct Engine {
             const int nrows = rows_per * nmem;
             const int grid = std::min(c->nsm, (nrows + xw::NWARP - 1) / xw::NWARP);
             Prof pr(c, K_X);
-            launch(early(nmem), kern, grid, xw::NWARP * 32, smem, c->stream, reinterpret_cast<const Member<float>*>(mem),
+            launch(early(c, nmem), kern, grid, xw::NWARP * 32, smem, c->stream, reinterpret_cast<const Member<float>*>(mem),
                    rl, reinterpret_cast<const cpx<float>*>(c->tw), rows_per, nrows);
             return after_launch(c, "row_nonlin_warp");
         } else if constexpr (MODE == RM_NONLIN && sizeof(T) == 4 && (N == 64 || N == 128 || N == 256)) {
@@ -530,7 +542,7 @@ struct Engine {
             const int nblk = nrows / Q;
             const int grid = std::min(c->nsm, (nblk + xwg::NWARP - 1) / xwg::NWARP);
             Prof pr(c, K_X);
-            launch(early(nmem), kern, grid, xwg::NWARP * 32, smem, c->stream, reinterpret_cast<const Member<float>*>(mem),
+            launch(early(c, nmem), kern, grid, xwg::NWARP * 32, smem, c->stream, reinterpret_cast<const Member<float>*>(mem),
                    rl, reinterpret_cast<const cpx<float>*>(c->tw), rows_per, nrows);
             return after_launch(c, "row_nonlin_wg");
         } else if constexpr (MODE == RM_NONLIN && rnl_fused<T, N>()) {
@@ -544,7 +556,7 @@ struct Engine {
             const int ntiles = tiles_per * nmem;
             const int grid = std::min(ntiles, c->nsm * rnl_ctas<T, N>());
             Prof pr(c, K_X);
-            launch(early(nmem), kern, grid, rnl_threads<T, N>(), smem, c->stream, mem, rl, (const C*)c->tw, tiles_per,
+            launch(early(c, nmem), kern, grid, rnl_threads<T, N>(), smem, c->stream, mem, rl, (const C*)c->tw, tiles_per,
                    ntiles);
             return after_launch(c, "row_nonlin");
         }
@@ -569,7 +581,7 @@ struct Engine {
         const int ntiles = tiles_per * nmem;
         const int grid = std::min(ntiles, c->nsm * ROW_CTAS);
         Prof pr(c, K_X);
-        launch(early(nmem), kern, grid, ROW_THREADS, smem, c->stream, mem, rl, (const C*)c->tw, tiles_per, ntiles);
+        launch(early(c, nmem), kern, grid, ROW_THREADS, smem, c->stream, mem, rl, (const C*)c->tw, tiles_per, ntiles);
         return after_launch(c, "row_pass");
     }
 
@@ -585,14 +597,14 @@ struct Engine {
         const int nblk = nrows / xr::rows<N>();
         const int grid = std::min(c->nsm, (nblk + xr::NWARP - 1) / xr::NWARP);
         Prof pr(c, K_X);
-        launch(early(nmem), kern, grid, xr::NWARP * 32, smem, c->stream, mem, rl, user,
+        launch(early(c, nmem), kern, grid, xr::NWARP * 32, smem, c->stream, mem, rl, user,
                reinterpret_cast<const cpx<float>*>(c->tw), N * N, nrows);
         return after_launch(c, "row_bulk");
     }
 
     static int symmetrize(bfg_ctx* c, const Mem* mem, int nmem, int bufi) {
         Prof pr(c, K_KSPACE);
-        launch(early(nmem), symmetrize_kernel<T, N>, dim3((N * N + 255) / 256, nmem), 256, 0, c->stream, mem, bufi);
+        launch(early(c, nmem), symmetrize_kernel<T, N>, dim3((N * N + 255) / 256, nmem), 256, 0, c->stream, mem, bufi);
         return after_launch(c, "symmetrize");
     }
 
@@ -2358,6 +2370,7 @@ static int ens_prepare(bfg_ens* e) {
         }
         g->launcher.stream = g->stream;
         g->launcher.tctr = g->tctr;
+        g->launcher.captured = e->use_graphs && sizes.size() == 1;
         for (int i : g->members) g->any_tracers = g->any_tracers || e->entries[i].tracers != nullptr;
         // member descriptors
         std::vector<unsigned char> host;
